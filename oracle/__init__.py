@@ -37,7 +37,7 @@ def build() -> None:
     binaries into _ref/ (kept when already built)."""
     subprocess.run(["make", "-s", "-C", HERE, "all"], check=True)
     refdir = os.environ.get("CDTW_REFERENCE_DIR", "")
-    if refdir and os.path.isdir(refdir) and not all(
+    if refdir and os.path.isfile(os.path.join(refdir, "include", "ldtw.cuh")) and not all(
             os.path.exists(os.path.join(REF_DIR, b))
             for b in ("UCR_DTW_BIN", "UCR_ED_BIN", "UCR_DTW", "ref_ldtw")):
         subprocess.run(["make", "-s", "-C", HERE, "ref", f"REFDIR={refdir}"], check=True)
