@@ -91,7 +91,7 @@ __device__ __forceinline__ double warp_scan_d(double v, int lane) {
 
 // Mean / sigma of the Tq windows of the tile staged in xs (Tq + M - 1
 // samples), FP64 sums with a per-warp shift slid 32 windows per round
-// (the avg_std kernel's scheme, from shared memory).
+// (the scheme of avg_std_long_kernel, from shared memory).
 __device__ void tile_stats(const float* xs, int Tq, int M, double* mu, float* sg) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int per = (Tq + kBatchWarps - 1) / kBatchWarps;

@@ -297,7 +297,7 @@ int cdtw_all_windows_host(cdtw_handle h, const float* h_query, int M, const floa
     float* dout = (float*)(base + o_out);
     CDTW_TRY(cdtw_set_query(h, h_query, M, W, CDTW_HOST));
     // pipeline over window chunks (multiples of the statistics kernel's
-    // 2048-window warp runs, so per-chunk statistics equal the whole-stream
+    // 2048-window tiles, so per-chunk statistics equal the whole-stream
     // ones): samples in on xfer[0], statistics + cDTW alternately on the
     // handle's stream and xfer[2] (a chunk's first waves overlap the previous
     // chunk's last), results out on xfer[1]; copies overlap compute

@@ -4,12 +4,13 @@
 // the whole stream (CUB scans, 2 cudaMalloc + 5 kernels per 1e7-sample epoch,
 // stats.cuh:85-142) and then takes the variance in FP32 (stats.cuh:49), which
 // loses the variance of level-shifted signals.  Here one kernel reads the
-// stream once: each warp owns a run of consecutive windows in four
-// sub-runs, keeps FP64 sums of (x-c) and (x-c)^2 for a shift c per sub-run,
-// and slides them 32 windows per round with warp scans of the
-// entering-minus-leaving terms (the four sub-runs' scans interleaved).
-// Output per window: mean (FP64) and sigma (FP32), 12 bytes.
+// stream once per tile of kTileWindows windows: FP64 sums of (x-c) and
+// (x-c)^2, c the tile's first sample, per chunk of eight samples, a block scan
+// over the chunks, and per thread eight windows slid from the difference of
+// two prefixes.  Output per window: mean (FP64) and sigma (FP32), 12 bytes.
 #include "common.cuh"
+
+#include <algorithm>
 
 namespace cdtw {
 
@@ -26,9 +27,11 @@ __device__ __forceinline__ double warp_sum(double v) {
     return v;
 }
 
+// Windows of any length, a warp per run of kStatsWarpWindows: serves the
+// lengths above kTileMaxM, whose tile would not fit shared memory.
 template <class XT, class ST>
 __global__ void __launch_bounds__(kStatsBlock)
-avg_std_kernel(const XT* __restrict__ x, int64_t N, int M, double* __restrict__ mu,
+avg_std_long_kernel(const XT* __restrict__ x, int64_t N, int M, double* __restrict__ mu,
                ST* __restrict__ sigma) {
     // The warp's run of kStatsWarpWindows windows is split into kStatsSub
     // sub-runs, each with its own shift c and starting sums; their scans are
@@ -113,6 +116,293 @@ avg_std_kernel(const XT* __restrict__ x, int64_t N, int M, double* __restrict__ 
             s2[u] += __shfl_sync(0xffffffffu, i2[u], 31);
         }
     }
+}
+
+// Deviation of a positive variance.  For the FP32 result: an FP32 estimate
+// (s0 = v * rsqrt(v)) and one Heron step whose residual v - s0^2 is taken in
+// FP64, so the result is the FP64 root rounded to FP32 but for ties within
+// 1e-7 ulp, at a fraction of the FP64 square root's instructions.
+__device__ __forceinline__ double std_of(double var, double) {
+    return var > 0.0 ? sqrt(var) : 1.0;
+}
+__device__ __forceinline__ float std_of(double var, float) {
+    const float v = (float)var;
+    if (!(v > 1e-30f && v < 1e30f)) return var > 0.0 ? (float)sqrt(var) : 1.0f;
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(v));
+    const float s0 = v * y;
+    const double s = (double)s0;
+    return fmaf((float)fma(-s, s, var), 0.5f * y, s0);
+}
+
+// One block per tile of kTileWindows windows, kTileR = 16 consecutive windows
+// per thread.  The tile's kTileWindows + M samples are staged in shared memory
+// with one 16-byte pad per 16 samples, so a warp's 16-byte accesses (lanes 16
+// samples apart) fall on all banks; chunk c holds samples 16c .. 16c+15.  The
+// sums of a thread's first window are the prefix at 16t + M (the chunk prefix
+// plus M mod 16 samples) less the prefix at 16t; the others follow by sliding,
+// the leaving samples still in registers.  Results go out through shared
+// memory in whole lines.
+//
+// Where the variance is below 2^-22 of the prefix it was taken from (over M:
+// 2^30 units in the prefix's last place; flat runs, a level shift inside the
+// tile) the difference of prefixes may have lost it, and a NaN or Inf sample
+// leaves the prefixes behind it without a value: such windows are summed again
+// about their own first sample, so a constant window has variance exactly 0
+// (sigma 1) wherever it lies and a bad sample spoils the windows that hold it
+// only.
+//
+// Bound: HBM (16 bytes a window, 82 us at 2^25 windows and 6546 GB/s) if the
+// latencies of a block's phases were hidden; 72 instructions a window, 24
+// warps per SM.  Six blocks per SM (80 registers, 100 bytes spilled) measured
+// best: 4 / 5 / 6 / 7 / 8 blocks 198 / 169 / 156 / 161 / 168 us at 2^25
+// windows, M = 512, and 10 us at 2^20 windows, M = 128.  Before (a warp per
+// 2048 windows, scans of 32 windows a round): 196 and 22 us, the latter the
+// latency of its serial rounds.
+constexpr int kTileThreads = 128;
+constexpr int kTileR = 16;                                // windows per thread, samples per chunk
+constexpr int kTileWindows = kTileThreads * kTileR;       // 2048
+constexpr int kTileMaxM = 8192;
+
+// Element i of an array of T with one 16-byte pad per 16 elements.
+template <class T>
+__host__ __device__ constexpr int tile_at(int i) {
+    return i + (int)(16 / sizeof(T)) * (i >> 4);
+}
+
+template <class XT, class ST>
+size_t tile_smem(int M) {
+    const int S = (int)round_up(kTileWindows + M, kTileR), NC = S / kTileR;
+    const size_t in = sizeof(XT) * (size_t)tile_at<XT>(S) + 2 * sizeof(double) * (size_t)NC;
+    return std::max(in, sizeof(double) * (size_t)tile_at<double>(kTileWindows));
+}
+
+// Elements 16c .. 16c+15 of a padded array, by 16-byte loads.
+__device__ __forceinline__ void tile_load16(const float* p, float (&v)[16]) {
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+        const float4 a = reinterpret_cast<const float4*>(p)[g];
+        v[4 * g] = a.x;
+        v[4 * g + 1] = a.y;
+        v[4 * g + 2] = a.z;
+        v[4 * g + 3] = a.w;
+    }
+}
+__device__ __forceinline__ void tile_load16(const double* p, double (&v)[16]) {
+#pragma unroll
+    for (int g = 0; g < 8; ++g) {
+        const double2 a = reinterpret_cast<const double2*>(p)[g];
+        v[2 * g] = a.x;
+        v[2 * g + 1] = a.y;
+    }
+}
+__device__ __forceinline__ void tile_store16(float* p, const float (&v)[16]) {
+#pragma unroll
+    for (int g = 0; g < 4; ++g)
+        reinterpret_cast<float4*>(p)[g] =
+            make_float4(v[4 * g], v[4 * g + 1], v[4 * g + 2], v[4 * g + 3]);
+}
+__device__ __forceinline__ void tile_store16(double* p, const double (&v)[16]) {
+#pragma unroll
+    for (int g = 0; g < 8; ++g)
+        reinterpret_cast<double2*>(p)[g] = make_double2(v[2 * g], v[2 * g + 1]);
+}
+
+// The 16 samples that enter thread t's windows, 16t + M .. 16t + M + 15: the
+// aligned vectors that cover them, shifted down by M mod V (the same for every
+// thread).
+__device__ __forceinline__ void tile_entering(const float* xs, int t, int M, float (&v)[16]) {
+    float y[20];
+    const int u0 = M & ~3;
+#pragma unroll
+    for (int g = 0; g < 5; ++g) {
+        const int u = min(u0 + 4 * g, ((M + 15) & ~3));
+        const float4 a = *reinterpret_cast<const float4*>(xs + 20 * t + tile_at<float>(u));
+        y[4 * g] = a.x;
+        y[4 * g + 1] = a.y;
+        y[4 * g + 2] = a.z;
+        y[4 * g + 3] = a.w;
+    }
+    const bool b1 = M & 1, b2 = M & 2;
+#pragma unroll
+    for (int k = 0; k < 18; ++k) y[k] = b2 ? y[k + 2] : y[k];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) v[k] = b1 ? y[k + 1] : y[k];
+}
+__device__ __forceinline__ void tile_entering(const double* xs, int t, int M, double (&v)[16]) {
+    double y[18];
+    const int u0 = M & ~1;
+#pragma unroll
+    for (int g = 0; g < 9; ++g) {
+        const int u = min(u0 + 2 * g, ((M + 15) & ~1));
+        const double2 a = *reinterpret_cast<const double2*>(xs + 18 * t + tile_at<double>(u));
+        y[2 * g] = a.x;
+        y[2 * g + 1] = a.y;
+    }
+    const bool b1 = M & 1;
+#pragma unroll
+    for (int k = 0; k < 16; ++k) v[k] = b1 ? y[k + 1] : y[k];
+}
+
+// Mean and variance of the window at tile sample i0, about its first sample.
+template <class XT>
+__device__ __noinline__ double2 tile_window(const XT* xs, int i0, int M) {
+    const double f = (double)xs[tile_at<XT>(i0)], invM = 1.0 / (double)M;
+    double a1 = 0.0, a2 = 0.0;
+    for (int k = 1; k < M; ++k) {
+        const double d = (double)xs[tile_at<XT>(i0 + k)] - f;
+        a1 += d;
+        a2 = fma(d, d, a2);
+    }
+    a1 *= invM;
+    return make_double2(f + a1, fma(-a1, a1, a2 * invM));
+}
+
+// The tile's n results, 16 of them in each thread's v, to out through z (16-byte
+// lines where out is aligned; the block's earlier accesses to z are done after
+// the first barrier).
+template <class T>
+__device__ __forceinline__ void tile_out(T* z, const T (&v)[kTileR], T* __restrict__ out, int n) {
+    constexpr int V = 16 / (int)sizeof(T);
+    const int t = threadIdx.x;
+    __syncthreads();
+    tile_store16(z + tile_at<T>(kTileR * t), v);
+    __syncthreads();
+    if (n == kTileWindows && (reinterpret_cast<uintptr_t>(out) & 15) == 0) {
+#pragma unroll
+        for (int i = V * t; i < kTileWindows; i += V * kTileThreads)
+            *reinterpret_cast<int4*>(out + i) = *reinterpret_cast<const int4*>(z + tile_at<T>(i));
+    } else {
+        for (int i = t; i < n; i += kTileThreads) out[i] = z[tile_at<T>(i)];
+    }
+}
+
+template <class XT, class ST>
+__global__ void __launch_bounds__(kTileThreads, 6)
+avg_std_kernel(const XT* __restrict__ x, int64_t N, int M, double* __restrict__ mu,
+               ST* __restrict__ sigma) {
+    extern __shared__ __align__(16) unsigned char tsm[];
+    constexpr int kWarps = kTileThreads / 32;
+    constexpr int V = 16 / (int)sizeof(XT);  // samples of a 16-byte vector
+    __shared__ double tot[2][kWarps];
+    const int64_t Nw = N - M + 1;
+    const int64_t t0 = (int64_t)blockIdx.x * kTileWindows;
+    const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+    const int S = (kTileWindows + M + kTileR - 1) / kTileR * kTileR, NC = S / kTileR;
+    XT* xs = (XT*)tsm;
+    double* C1 = (double*)(xs + tile_at<XT>(S));
+    double* C2 = C1 + NC;
+    const XT* __restrict__ xt = x + t0;
+    const XT first = xt[0];
+    const double c = (double)first;
+    // samples past the stream enter windows that are not stored only
+    const int have = (int)min((int64_t)S, N - t0);
+    int i0 = 0;
+    if ((reinterpret_cast<uintptr_t>(x) & 15) == 0) {  // t0 is a multiple of 2048
+        i0 = have / V * V;
+        for (int i = V * t; i < i0; i += V * kTileThreads)
+            *reinterpret_cast<int4*>(xs + tile_at<XT>(i)) =
+                *reinterpret_cast<const int4*>(xt + i);
+    }
+    for (int i = i0 + t; i < S; i += kTileThreads) xs[tile_at<XT>(i)] = i < have ? xt[i] : first;
+    __syncthreads();
+    // chunk sums and their exclusive prefix, kTileThreads chunks a round
+    double v[kTileR];  // the thread's own chunk, about c
+    double base1 = 0.0, base2 = 0.0;
+    for (int r0 = 0; r0 < NC; r0 += kTileThreads) {
+        if (r0) __syncthreads();  // the previous round's totals are read
+        const int ch = r0 + t;
+        double e1 = 0.0, e2 = 0.0;
+        if (r0 + 32 * wid < NC) {  // whole warps
+            double a1 = 0.0, a2 = 0.0;
+            XT xv[kTileR];
+            tile_load16(xs + (kTileR + V) * min(ch, NC - 1), xv);
+            if (ch < NC) {
+#pragma unroll
+                for (int k = 0; k < kTileR; ++k) {
+                    const double d = (double)xv[k] - c;
+                    if (r0 == 0) v[k] = d;
+                    a1 += d;
+                    a2 = fma(d, d, a2);
+                }
+            }
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const double u1 = __shfl_up_sync(0xffffffffu, a1, o);
+                const double u2 = __shfl_up_sync(0xffffffffu, a2, o);
+                if (lane >= o) {
+                    a1 += u1;
+                    a2 += u2;
+                }
+            }
+            e1 = __shfl_up_sync(0xffffffffu, a1, 1);
+            e2 = __shfl_up_sync(0xffffffffu, a2, 1);
+            if (lane == 0) e1 = e2 = 0.0;
+            if (lane == 31) {
+                tot[0][wid] = a1;
+                tot[1][wid] = a2;
+            }
+        } else if (lane == 31) {
+            tot[0][wid] = tot[1][wid] = 0.0;
+        }
+        __syncthreads();
+        double b1 = base1, b2 = base2;
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) {
+            const double u1 = tot[0][w], u2 = tot[1][w];
+            b1 += w < wid ? u1 : 0.0;
+            b2 += w < wid ? u2 : 0.0;
+            base1 += u1;
+            base2 += u2;
+        }
+        if (ch < NC) {
+            C1[ch] = b1 + e1;
+            C2[ch] = b2 + e2;
+        }
+    }
+    __syncthreads();
+    // sums of the thread's first window
+    const int e = kTileR * t + M, ce = e / kTileR, rest = e % kTileR;
+    double w1 = C1[ce], w2 = C2[ce];
+    for (int k = 0; k < rest; ++k) {
+        const double d = (double)xs[(kTileR + V) * ce + k] - c;
+        w1 += d;
+        w2 = fma(d, d, w2);
+    }
+    const double invM = 1.0 / (double)M;
+    const double lost = w2 * invM * 0x1p-22;
+    w1 -= C1[t];
+    w2 -= C2[t];
+    XT in[kTileR];
+    tile_entering(xs, t, M, in);
+    double om[kTileR];
+    ST os[kTileR];
+    unsigned again = 0;  // windows to be summed again
+#pragma unroll
+    for (int r = 0; r < kTileR; ++r) {
+        const double m1 = w1 * invM;
+        const double var = fma(-m1, m1, w2 * invM);
+        om[r] = c + m1;
+        os[r] = std_of(var, ST());
+        again |= var >= lost ? 0u : 1u << r;
+        const double vin = (double)in[r] - c, d = vin - v[r];
+        w1 += d;
+        w2 = fma(d, vin + v[r], w2);
+    }
+    if (again) {
+#pragma unroll
+        for (int r = 0; r < kTileR; ++r) {
+            if ((again >> r & 1u) && t0 + kTileR * t + r < Nw) {
+                const double2 q = tile_window(xs, kTileR * t + r, M);
+                om[r] = q.x;
+                os[r] = std_of(q.y, ST());
+            }
+        }
+    }
+    // the samples and prefixes make room for the sigmas, these for the means
+    tile_out(reinterpret_cast<ST*>(tsm), os, sigma + t0, (int)min((int64_t)kTileWindows, Nw - t0));
+    tile_out(reinterpret_cast<double*>(tsm), om, mu + t0,
+             (int)min((int64_t)kTileWindows, Nw - t0));
 }
 
 // One block prepares the query pack: FP64 two-pass z-normalisation (the
@@ -220,30 +510,37 @@ prepare_queries_kernel(const float* __restrict__ raw, const int64_t* __restrict_
 
 }  // namespace
 
-int launch_avg_std(cdtw_handle h, const float* x, int64_t N, int M, double* mu, float* sigma) {
+template <class XT, class ST>
+static int launch_stats(cdtw_handle h, const XT* x, int64_t N, int M, double* mu, ST* sigma) {
     const int64_t Nw = N - M + 1;
-    const int64_t warps = div_up(Nw, kStatsWarpWindows);
-    const int64_t blocks = div_up(warps, kStatsBlock / 32);
-    avg_std_kernel<float, float><<<(unsigned)blocks, kStatsBlock, 0, h->stream>>>(x, N, M, mu,
-                                                                                  sigma);
+    if (M > kTileMaxM) {
+        const int64_t blocks = div_up(div_up(Nw, kStatsWarpWindows), kStatsBlock / 32);
+        avg_std_long_kernel<XT, ST><<<(unsigned)blocks, kStatsBlock, 0, h->stream>>>(x, N, M, mu,
+                                                                                    sigma);
+        CDTW_LAUNCH(h, "avg_std_long_kernel");
+        return CDTW_OK;
+    }
+    const size_t smem = tile_smem<XT, ST>(M);
+    if (smem > 48 * 1024)
+        CDTW_CUDA(h, cudaFuncSetAttribute((const void*)avg_std_kernel<XT, ST>,
+                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)smem));
+    avg_std_kernel<XT, ST><<<(unsigned)div_up(Nw, kTileWindows), kTileThreads, smem, h->stream>>>(
+        x, N, M, mu, sigma);
     CDTW_LAUNCH(h, "avg_std_kernel");
     return CDTW_OK;
 }
 
+int launch_avg_std(cdtw_handle h, const float* x, int64_t N, int M, double* mu, float* sigma) {
+    return launch_stats(h, x, N, M, mu, sigma);
+}
+
 // FP64 sigma (ED and LDTW paths), float32 or float64 series.
 int launch_avg_std64(cdtw_handle h, const float* x, int64_t N, int M, double* mu, double* sigma) {
-    const int64_t blocks = div_up(div_up(N - M + 1, kStatsWarpWindows), kStatsBlock / 32);
-    avg_std_kernel<float, double><<<(unsigned)blocks, kStatsBlock, 0, h->stream>>>(x, N, M, mu,
-                                                                                   sigma);
-    CDTW_LAUNCH(h, "avg_std_kernel");
-    return CDTW_OK;
+    return launch_stats(h, x, N, M, mu, sigma);
 }
 int launch_avg_std64(cdtw_handle h, const double* x, int64_t N, int M, double* mu, double* sigma) {
-    const int64_t blocks = div_up(div_up(N - M + 1, kStatsWarpWindows), kStatsBlock / 32);
-    avg_std_kernel<double, double><<<(unsigned)blocks, kStatsBlock, 0, h->stream>>>(x, N, M, mu,
-                                                                                    sigma);
-    CDTW_LAUNCH(h, "avg_std_kernel");
-    return CDTW_OK;
+    return launch_stats(h, x, N, M, mu, sigma);
 }
 
 int launch_prepare_queries(cdtw_handle h, const float* raw, const int64_t* offs,
