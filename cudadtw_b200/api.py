@@ -377,7 +377,7 @@ class Handle:
         ``path`` (a uint8 device buffer of pair_path_bytes) the optimal path is
         recorded for pair_bwd; ``mode`` "store" (2-bit directions) or
         "recompute" (checkpoints, segments recomputed during the walk), None
-        for the library's choice by memory."""
+        for the library's choice by memory and speed."""
         _dev(q, torch.float32, "q")
         _dev(s, torch.float32, "s")
         if q.shape != s.shape or q.dim() != 2:

@@ -777,7 +777,8 @@ int cdtw_pair_fwd(cdtw_handle h, const float* d_q, const float* d_s, int64_t n, 
     size_t o_zq, o_zs, o_dirs;
     CDTW_TRY(ensure_workspace(
         h, pair_carve(n, L, W, flags, d_path != nullptr, recompute, &o_zq, &o_zs, &o_dirs)));
-    h->last_pair_recompute = recompute ? 1 : 0;
+    const bool store = flags & CDTW_PAIR_STORE_DIRS;
+    h->last_pair_recompute = d_path && (recompute || (!store && pair_auto_mode(L, W) != 0)) ? 1 : 0;
     char* ws = (char*)h->ws;
     double* hdr = (double*)d_path;
     uint32_t* rows = d_path ? (uint32_t*)((char*)d_path + (size_t)n * 32) : nullptr;
@@ -794,7 +795,8 @@ int cdtw_pair_fwd(cdtw_handle h, const float* d_q, const float* d_s, int64_t n, 
         return launch_pair_fwd_ckpt(h, zq, zs, n, L, W, metric == CDTW_EUCLIDEAN, d_D,
                                     (float*)(ws + o_dirs), rows, cols);
     return launch_pair_fwd(h, zq, zs, n, L, W, metric == CDTW_EUCLIDEAN, d_D,
-                           d_path ? (uint32_t*)(ws + o_dirs) : nullptr, rows, cols);
+                           d_path ? (uint32_t*)(ws + o_dirs) : nullptr, rows, cols, -1, nullptr,
+                           0, -1, false, store);
 }
 
 int cdtw_pair_last_mode(cdtw_handle h, int* recompute) {

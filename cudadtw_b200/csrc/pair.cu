@@ -43,6 +43,7 @@ __global__ void pair_znorm_kernel(const float* __restrict__ q, const float* __re
 }
 
 constexpr int kBwdThreads = 128;
+constexpr int kCorridorC = 4;  // slots per lane of the corridor walk (5 for segments of 128)
 
 // Block-wide FP64 sums of a and b (every thread gets them); blocks of 1 to 4
 // warps; red holds 2 x 4 doubles.
@@ -291,6 +292,34 @@ size_t pair_ckpt_floats(int L, int W) {
     return (size_t)pair_ckpt_nseg(L, W, C) * 2 * C * G;
 }
 
+// Segments and floats of thin checkpoints per pair (two anti-diagonals every
+// thin_seg(C) after the first: the W + 1 band slots alone, or all G x C for
+// wide lanes).
+static int pair_thin_nseg(int L, int W, int C) {
+    const int K = 2 * L - 1, k0 = (W & 1) ? 2 : 1;
+    return (int)std::max<int64_t>(1, div_up(std::max(K - k0, 1), thin_seg(C)));
+}
+static size_t pair_thin_floats(int L, int W, int G, int C) {
+    return (size_t)(pair_thin_nseg(L, W, C) - 1) * 2 * (C <= kThinBody ? W + 1 : C * G);
+}
+
+// How a forward with a path record and scratch for stored directions records
+// it: 0 direction bits, 1 thin checkpoints, 2 wide ones, in that scratch.  The
+// checkpointed walks recompute a corridor of the band only, which costs less
+// than direction bits for all of it: 4096 pairs of 512, W = 51, 288 us with
+// bits and 251 with thin checkpoints, 512 of 2048, W = 409, 1460 / 483 and 612
+// with wide ones.  Thin ones need their floats to fit the bits' scratch, which
+// leaves out bands within 1/16 of a power-of-two group's full width and
+// W >= 480; wide ones serve those of W >= 128.
+int pair_auto_mode(int L, int W) {
+    int G, C;
+    pair_shape(L, W, &G, &C);
+    const size_t words = pair_dirs_words(L, W);
+    if (words == 0 || C < 2 || C > 16) return 0;
+    if (thin_seg(C) <= kThinSeg && pair_thin_floats(L, W, G, C) <= words) return 1;
+    return C > kCorridorC && pair_ckpt_floats(L, W) <= words ? 2 : 0;
+}
+
 int launch_pair_znorm(cdtw_handle h, const float* q, const float* s, int64_t n, int L, float* zq,
                       float* zs, double* hdr) {
     const int64_t warps = 2 * n;
@@ -303,10 +332,13 @@ int launch_pair_znorm(cdtw_handle h, const float* q, const float* s, int64_t n, 
 int launch_pair_fwd(cdtw_handle h, const float* zq, const float* zs, int64_t n, int L, int W,
                     bool euclid, float* D, uint32_t* dirs, uint32_t* rows, uint32_t* cols,
                     int64_t qstride, const int* gate, int gate_max, int gate_min,
-                    bool wide) {
+                    bool wide, bool store) {
     int G, C;
     pair_shape(L, W, &G, &C);
     if (C > 16) return set_error(h, CDTW_EUNSUPPORTED, "pair band W=%d exceeds 511", W);
+    const int mode = rows && cols && dirs && !store ? pair_auto_mode(L, W) : 0;
+    if (mode == 2)
+        return launch_pair_fwd_ckpt(h, zq, zs, n, L, W, euclid, D, (float*)dirs, rows, cols);
     if (!rows && wide) {
         G = 32;
         C = (W + 1 + G - 1) / G;
@@ -339,13 +371,19 @@ int launch_pair_fwd(cdtw_handle h, const float* zq, const float* zs, int64_t n, 
     a.ckpt = nullptr;
     a.seg = 0;
     a.nseg = 0;
+    a.C = C;
     const int threads = kPairThreads;
     const int64_t groups_per_block = threads / G;
     // a path is recorded when the run arrays are given; the direction scratch
     // is needed only outside shared-record mode
     size_t shared_rec;
     const bool shared = pair_shared_record(L, G, C, &a.recb, &a.logb, &shared_rec);
-    const int dm = !rows ? 0 : shared ? 2 : 1;
+    const int dm = !rows ? 0 : shared ? 2 : mode == 1 ? 5 : 1;
+    if (dm == 5) {
+        a.ckpt = (float*)dirs;
+        a.seg = thin_seg(C);
+        a.nseg = pair_thin_nseg(L, W, C);
+    }
     if (dm != 0 && !cols) return set_error(h, CDTW_EINVAL, "path record without column runs");
     if (dm == 1 && !dirs) return set_error(h, CDTW_EINVAL, "path record without direction scratch");
     // DM 1: backtracking ring (kWalkStages chunks of kWalkChunk bytes per lane)
@@ -361,6 +399,14 @@ int launch_pair_fwd(cdtw_handle h, const float* zq, const float* zs, int64_t n, 
                                       (int)smem));
     k<<<(int)blocks, threads, smem, h->stream>>>(a);
     CDTW_LAUNCH(h, "pair_fwd_kernel");
+    if (dm == 5) {
+        const unsigned warps = kPairThreads / 32;
+        if (euclid)
+            pair_thin_kernel<true><<<(unsigned)div_up(n, warps), kPairThreads, 0, h->stream>>>(a);
+        else
+            pair_thin_kernel<false><<<(unsigned)div_up(n, warps), kPairThreads, 0, h->stream>>>(a);
+        CDTW_LAUNCH(h, "pair_thin_kernel");
+    }
     return CDTW_OK;
 }
 
@@ -396,23 +442,31 @@ int launch_pair_fwd_ckpt(cdtw_handle h, const float* zq, const float* zs, int64_
     a.ckpt = ckpt;
     a.seg = pair_ckpt_seg(C);
     a.nseg = pair_ckpt_nseg(L, W, C);
+    a.C = C;
     const int threads = kPairThreads;
     const int64_t groups_per_block = threads / G;
     const int64_t blocks = div_up(n, groups_per_block);
     if (blocks > INT32_MAX) return set_error(h, CDTW_EINVAL, "too many pairs");
-    const int eb = C <= 4 ? 1 : (C <= 8 ? 2 : 4);
+    const bool corridor = C > kCorridorC;  // then G = 32
+    const int wide = a.seg + 1 > 32 * kCorridorC ? 1 : 0;
+    const int eb = corridor ? 1 + wide : 1;
     // records of the longest segment (segment 0 holds up to seg + 2 rows)
     a.recb = (int)round_up((int64_t)(a.seg + 2) * G * eb, 128) + 32;
     a.logb = (int)round_up(a.seg + 2, 128) + 32;
     const PairFwdK kf = fwd_kernel(C, euclid, 3);
     kf<<<(int)blocks, threads, 0, h->stream>>>(a);
     CDTW_LAUNCH(h, "pair_fwd_kernel");
-    const PairFwdK kw = fwd_kernel(C, euclid, 4);
+    const PairFwdK kw =
+        !corridor ? fwd_kernel(C, euclid, 4)
+        : wide    ? (euclid ? pair_corridor_kernel<kCorridorC + 1, true>
+                            : pair_corridor_kernel<kCorridorC + 1, false>)
+                  : (euclid ? pair_corridor_kernel<kCorridorC, true>
+                            : pair_corridor_kernel<kCorridorC, false>);
     const size_t smem = (size_t)groups_per_block * (size_t)(a.recb + a.logb);
     CDTW_CUDA(h, cudaFuncSetAttribute((const void*)kw, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)smem));
     kw<<<(int)blocks, threads, smem, h->stream>>>(a);
-    CDTW_LAUNCH(h, "pair_ckpt_walk_kernel");
+    CDTW_LAUNCH(h, corridor ? "pair_corridor_kernel" : "pair_ckpt_walk_kernel");
     return CDTW_OK;
 }
 

@@ -345,9 +345,9 @@ size_t cdtw_pair_path_bytes(int64_t n, int L);
 
 /* Device work memory cdtw_pair_fwd takes from the handle's grow-only workspace
  * for n pairs: z-normalised copies of both series (flags & CDTW_PAIR_ZNORM)
- * and, when a path is recorded (with_path != 0), either 2 bits per band cell
- * of predecessor choices, padded to the lane layout, or (recomputation) two
- * anti-diagonals of the band every ~128 anti-diagonals.  The mode is that of
+ * and, when a path is recorded (with_path != 0), either the room of 2 bits per
+ * band cell of predecessor choices, padded to the lane layout, or
+ * (recomputation) two anti-diagonals of the band every ~128 anti-diagonals.  The mode is that of
  * cdtw_pair_fwd without a memory limit on the handle.  0 for invalid sizes. */
 size_t cdtw_pair_workspace_bytes(int64_t n, int L, int W, int flags, int with_path);
 
@@ -357,10 +357,12 @@ size_t cdtw_pair_workspace_bytes(int64_t n, int L, int W, int flags, int with_pa
  * back.  Recomputation from checkpoints: the forward keeps only two
  * anti-diagonals every ~128 (about 4x less scratch at L = 2048, W = 409),
  * and the walk recomputes each segment, last first, with its direction bits
- * in shared memory: the same path, bit for bit, for a second pass over the
- * band.  CDTW_PAIR_STORE_DIRS / CDTW_PAIR_RECOMPUTE force a mode; without
- * either, directions are stored unless their scratch would exceed 4 GiB (or
- * half the handle's memory limit).  No reference counterpart (the DP of
+ * in shared memory (of bands W >= 128 only the slots the path can reach): the
+ * same path, bit for bit.  CDTW_PAIR_STORE_DIRS / CDTW_PAIR_RECOMPUTE force a
+ * mode; without either, the scratch of stored directions is taken unless it
+ * would exceed 4 GiB (or half the handle's memory limit), and holds either
+ * those or, where that is faster, checkpoints as close as fit it, from which
+ * the path's surroundings are recomputed.  No reference counterpart (the DP of
  * include/cdtw.cuh:24-88 returns distances only). */
 
 /* 1 when the last cdtw_pair_fwd with a path record on this handle recomputed
