@@ -17,7 +17,7 @@ __global__ void __launch_bounds__(kBatchThreads)
 batch_reg_kernel(const BatchArgs b) {
     extern __shared__ __align__(16) unsigned char smem[];
     const TileSmem ts = carve_tile(smem, b.tmax, b.mmax);
-    float4* sq4 = ts.tail;                             // 4 * lq4max
+    float4* sq4 = ts.tail;                             // lq4max (of 4 * lq4max)
     float2* senv = (float2*)(sq4 + 4 * b.lq4max);      // mmax
     __shared__ int s_item, s_na, s_nb, s_next;
     const int tid = threadIdx.x, lane = tid & 31;
@@ -26,7 +26,7 @@ batch_reg_kernel(const BatchArgs b) {
         if (tid == 0) s_na = s_nb = s_next = 0;
         const BatchQ& Q = b.qs[q];
         const int M = Q.sa.M;
-        for (int e = tid; e < 4 * Q.lq4; e += kBatchThreads) sq4[e] = Q.qpad4[e];
+        for (int e = tid; e < Q.lq4; e += kBatchThreads) sq4[e] = Q.qpad4[e];
         for (int e = tid; e < M; e += kBatchThreads) senv[e] = Q.env[e];
         const int t0 = tile * Q.T;
         const int Tq = min(Q.T, Q.Nw - t0);
@@ -44,7 +44,7 @@ batch_reg_kernel(const BatchArgs b) {
             const Norm nm = make_norm(ts.mu[l], ts.sg[l]);
             const float lbk = (i < nb) ? ts.lb_k[i] : 0.f;
             const float res =
-                reg_window_dtw<W, EU>(sq4, Q.lq4, senv, M, b.x + t0 + l, nm, lbk, alive, Q.key);
+                reg_window_dtw<W, EU>(sq4, senv, M, b.x + t0 + l, nm, lbk, alive, Q.key);
             if (i < nb && res < CDTW_INF) atomicMin(Q.key, pack_key(res, (uint32_t)(t0 + l)));
         }
     }

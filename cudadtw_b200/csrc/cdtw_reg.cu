@@ -1,21 +1,5 @@
-// Banded DTW with the whole band of one window in registers ("register band").
-//
-// Reference: sparse_block_cdtw / dense_block_cdtw (include/cdtw.cuh:164-363),
-// which spread one window over W+2 threads and step the anti-diagonals through
-// shared memory with a __syncthreads per step.  Windows are independent and
-// there are millions of them, so here one thread owns one window and keeps
-// the 2W+1 band cells of the current row in registers; the 32 lanes of a warp
-// run 32 neighbouring windows in lockstep, so all lanes read the same query
-// values (a shared-memory broadcast) and consecutive stream samples (one
-// coalesced 128-byte load per row).
-//
-// Orientation: rows are window (data) positions j = 0..M-1, columns are query
-// positions i, band coordinate k = i - j + W in [0, 2W].  The cell update
-//   D[j][k] = cost(z_j, q_{j-W+k}) + min(D[j-1][k], D[j-1][k+1], D[j][k-1])
-// is one FADD, one three-input FMNMX and one FFMA.  Query positions outside
-// [0, M) are padded with +inf, which makes out-of-matrix cells +inf without
-// any per-cell test.  The result D[M-1][W] equals the reference's
-// penalty[...][M] (cdtw.cuh:83).
+// Launchers and kernel choice of the register-band cDTW; the device code and
+// its description are in cdtw_reg.cuh.
 #include "cdtw_reg.cuh"
 
 namespace cdtw {
@@ -27,12 +11,10 @@ struct RegKernels {
     RegKernel mh[kMaxRegW + 1];
     RegSearchKernel seu[kMaxRegW + 1];
     RegSearchKernel smh[kMaxRegW + 1];
-    RegKernel eu2[kMaxReg2W + 1];  // two windows per thread
-    RegKernel mh2[kMaxReg2W + 1];
-    RegKernel eu4[kMaxReg4W + 1];  // four windows per thread
-    RegKernel mh4[kMaxReg4W + 1];
-    RegCKernel euc[kMaxReg2W + 1];  // consecutive windows, all of them
-    RegCKernel mhc[kMaxReg2W + 1];
+    RegKernel eun[kMaxReg2W + 1];  // several windows per thread
+    RegKernel mhn[kMaxReg2W + 1];
+    RegCKernel euc[kMaxRegW + 1];  // consecutive windows, all of them
+    RegCKernel mhc[kMaxRegW + 1];
     RegKernels() {
         void** a = (void**)eu;
         void** b = (void**)mh;
@@ -44,12 +26,12 @@ struct RegKernels {
         reg_fill_part3(a, b, c, d);
         reg_fill_part4(a, b, c, d);
         reg_fill_part5(a, b, c, d);
-        reg2_fill_part0((void**)eu2, (void**)mh2);
-        reg2_fill_part1((void**)eu2, (void**)mh2);
-        reg4_fill_part0((void**)eu4, (void**)mh4);
+        regn_fill_part0((void**)eun, (void**)mhn);
         regc_fill_part0((void**)euc, (void**)mhc);
         regc_fill_part1((void**)euc, (void**)mhc);
         regc_fill_part2((void**)euc, (void**)mhc);
+        regc_fill_part3((void**)euc, (void**)mhc);
+        regc_fill_part4((void**)euc, (void**)mhc);
     }
 };
 
@@ -97,7 +79,7 @@ int launch_cdtw_search(cdtw_handle h, const float* x, int64_t N, const double* m
                                         sink);
     RegSearchKernel k = euclid ? reg_kernels().seu[q.W] : reg_kernels().smh[q.W];
     const int lq4 = q.lq / 4;
-    const size_t smem = (size_t)q.lq * 4 * sizeof(float) + (size_t)q.M * sizeof(float2);
+    const size_t smem = (size_t)q.lq * sizeof(float) + (size_t)q.M * sizeof(float2);
     CDTW_CUDA(h, cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)smem));
     int per_sm = 0;
@@ -128,36 +110,36 @@ int launch_cdtw_windows(cdtw_handle h, const float* x, int64_t N, const double* 
                                  variant == CDTW_VARIANT_STRIP16 ? 16 : 32, out);
     }
     if (L <= 0) return CDTW_OK;
-    // four windows per thread up to W = kMaxReg4W, two up to kMaxReg2W
-    // (register budget)
-    const int per = q.W <= kMaxReg4W ? 4 : (q.W <= kMaxReg2W ? 2 : 1);
     const int lq4 = q.lq / 4;
-    const size_t smem = (size_t)q.lq * 4 * sizeof(float);
-    if (!idx && per > 1 && L == Nw) {
+    const size_t smem = (size_t)q.lq * sizeof(float);
+    auto prepare = [&](const void* k) -> int {
+        if (smem > 48 * 1024)
+            CDTW_CUDA(h, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              (int)smem));
+        return CDTW_OK;
+    };
+    if (!idx && L == Nw) {
         // every window: the consecutive-window kernels (one sliding run of
         // the stream per thread)
         RegCKernel kc = euclid ? reg_kernels().euc[q.W] : reg_kernels().mhc[q.W];
-        if (smem > 48 * 1024)
-            CDTW_CUDA(h, cudaFuncSetAttribute((const void*)kc,
-                                              cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              (int)smem));
-        const unsigned blocks =
-            (unsigned)div_up(div_up(L, regc_per_thread(q.W)), kRegBlock);
+        CDTW_TRY(prepare((const void*)kc));
+        const unsigned blocks = (unsigned)div_up(div_up(L, reg_per_thread(q.W)), kRegBlock);
         kc<<<blocks, kRegBlock, smem, h->stream>>>(x, mu, sigma, (const float4*)q.qpad, lq4, q.M,
                                                    Nw, out);
         CDTW_LAUNCH(h, "cdtw_regc_kernel");
         return CDTW_OK;
     }
-    RegKernel k = per == 4   ? (euclid ? reg_kernels().eu4[q.W] : reg_kernels().mh4[q.W])
-                  : per == 2 ? (euclid ? reg_kernels().eu2[q.W] : reg_kernels().mh2[q.W])
-                             : (euclid ? reg_kernels().eu[q.W] : reg_kernels().mh[q.W]);
-    if (smem > 48 * 1024)
-        CDTW_CUDA(h, cudaFuncSetAttribute((const void*)k,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)smem));
-    const unsigned blocks = (unsigned)div_up(div_up(L, per), kRegBlock);
-    k<<<blocks, kRegBlock, smem, h->stream>>>(x, mu, sigma, (const float4*)q.qpad, lq4, q.M, Nw,
-                                              idx, (int)L, out);
+    // listed windows: several per thread when that still gives every scheduler
+    // a warp, else one, in blocks of a warp
+    const int per = reg_per_thread(q.W);
+    const bool many = per > 1 && L >= (int64_t)per * 128 * h->sm_count;
+    RegKernel k = many ? (euclid ? reg_kernels().eun[q.W] : reg_kernels().mhn[q.W])
+                       : (euclid ? reg_kernels().eu[q.W] : reg_kernels().mh[q.W]);
+    CDTW_TRY(prepare((const void*)k));
+    const int threads = L >= (int64_t)128 * h->sm_count ? kRegBlock : 32;
+    const unsigned blocks = (unsigned)div_up(div_up(L, many ? per : 1), threads);
+    k<<<blocks, threads, smem, h->stream>>>(x, mu, sigma, (const float4*)q.qpad, lq4, q.M, Nw,
+                                            idx, (int)L, out);
     CDTW_LAUNCH(h, "cdtw_reg_kernel");
     return CDTW_OK;
 }

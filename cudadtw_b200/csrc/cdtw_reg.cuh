@@ -16,6 +16,23 @@
 // [0, M) are padded with +inf, which makes out-of-matrix cells +inf without
 // any per-cell test.  The result D[M-1][W] equals the reference's
 // penalty[...][M] (cdtw.cuh:83).
+//
+// What bounds a cell is the register file: about two operands a cycle and
+// scheduler (measured: FFMA with two distinct registers 1.07 cycles a warp,
+// with three 1.60; FADD + two-input FMNMX + FFMA 3.26, with a three-input
+// FMNMX 4.13), and 4.2 is what a row at a time ran at.  So four rows go
+// together, each a cell behind the one above (reg_rows4): rows j .. j+3 then
+// stand on the same query value q_{j-W+s} at step s, a row's diagonal and upper
+// inputs are the two newest values of the row above, still in registers, and
+// the differences z - q of two neighbouring steps come from one packed
+// subtraction (z twice, the query pair as loaded).  A group of four rows loads
+// the query once, from one copy of it.  All windows, M = 128, in cycles a warp
+// and computed cell (2^22 windows: us), row at a time -> now: W = 12 4.19 ->
+// 3.87 (1395), W = 25 4.19 -> 3.77 (2773), W = 55 3.69 now.  Scalar
+// subtractions 4.2 to 4.4; rows in pairs 3.95 to 3.99, in eights 3.84 to 3.89;
+// the pair over rows instead of steps 3.96 to 4.08; subtraction and
+// multiply-add packed over two windows 4.7 to 5.1 (the three minimum operands
+// then share a register bank).
 #pragma once
 
 #include "common.cuh"
@@ -29,270 +46,160 @@ namespace {
 constexpr int kRegBlock = 128;
 constexpr int kMaxRegW = 96;
 
-template <int W, bool EU>
-__global__ void __launch_bounds__(kRegBlock)
+// (x, y) as a packed FP32 pair, and the two differences of two pairs.
+__device__ __forceinline__ unsigned long long pack2(float x, float y) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+    return r;
+}
+__device__ __forceinline__ void sub2(unsigned long long a, unsigned long long b, float& lo,
+                                     float& hi) {
+    unsigned long long r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(r));
+}
+
+// Rows j .. j+3 of NW windows: p holds row j-1 (p[v][B] = +inf) and becomes
+// row j+3; z[v][r] is window v's sample of row j + r, qr the padded query from
+// element j (16-byte aligned; reads up to 2W + 7 further).  Step s takes row r
+// to its cell s - r, whose query value is element s for every row.  CAP: res[v]
+// takes D[j + last][W] for last in 0..3.
+template <int W, bool EU, int NW, bool CAP>
+__device__ __forceinline__ void reg_rows4(float (&p)[NW][2 * W + 2], const float (&z)[NW][4],
+                                          const float4* qr, int last, float (&res)[NW]) {
+    constexpr int B = 2 * W + 1;
+    constexpr int kSteps = B + 3;
+    float l[NW][4], d1[NW][4];  // rows' newest cells and the ones before
+#pragma unroll
+    for (int v = 0; v < NW; ++v) {
+#pragma unroll
+        for (int r = 0; r < 4; ++r) l[v][r] = d1[v][r] = CDTW_INF;
+    }
+#pragma unroll
+    for (int s4 = 0; s4 < (kSteps + 3) / 4; ++s4) {
+        const float4 q4 = qr[s4];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const unsigned long long q2 = h ? pack2(q4.z, q4.w) : pack2(q4.x, q4.y);
+            float df[NW][4][2];
+#pragma unroll
+            for (int v = 0; v < NW; ++v) {
+#pragma unroll
+                for (int r = 0; r < 4; ++r)
+                    sub2(pack2(z[v][r], z[v][r]), q2, df[v][r][0], df[v][r][1]);
+            }
+#pragma unroll
+            for (int g = 0; g < 2; ++g) {
+                const int s = 4 * s4 + 2 * h + g;
+#pragma unroll
+                for (int v = 0; v < NW; ++v) {
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) {
+                        const int k = s - r;  // row j + r's cell
+                        if (k >= 0 && k < B) {
+                            const float diag = r == 0 ? p[v][k < B ? k : 0] : d1[v][r > 0 ? r - 1 : 0];
+                            const float up = r == 0 ? p[v][k < B ? k + 1 : B]
+                                                    : (k + 1 < B ? l[v][r > 0 ? r - 1 : 0] : CDTW_INF);
+                            const float c = cell<EU>(df[v][r][g], min3f(diag, l[v][r], up));
+                            d1[v][r] = l[v][r];
+                            l[v][r] = c;
+                            if (r == 3) p[v][k] = c;
+                            if (CAP && k == W) res[v] = r == last ? c : res[v];
+                        } else if (k == B) {
+                            d1[v][r] = l[v][r];  // the row below's last diagonal
+                        }
+                    }
+                }
+            }
+        }
+    }
+}
+
+template <int W, int NW>
+__device__ __forceinline__ void reg_init(float (&p)[NW][2 * W + 2]) {
+#pragma unroll
+    for (int v = 0; v < NW; ++v) {
+#pragma unroll
+        for (int k = 0; k <= 2 * W + 1; ++k) p[v][k] = CDTW_INF;
+        p[v][W] = 0.0f;  // virtual D[-1][-1] = 0 (cdtw.cuh:35, :191)
+    }
+}
+
+// Windows per thread: as many as the shortest rows need to overlap their
+// chains, no more (cycles a cell with 1 / 2 / 3 windows: W = 6 4.6 / 4.15 /
+// 3.99, W = 12 4.32 / 3.87 / 3.89, W = 25 3.84 / 3.77 / 3.79, W = 30 3.76 /
+// 3.82, W = 46 3.72 / 3.78): fewer registers leave more warps to a scheduler
+// and a finer split of short streams.
+constexpr int kMaxReg3W = 7;
+constexpr int kMaxReg2W = 28;
+constexpr int reg_per_thread(int W) { return W <= kMaxReg3W ? 3 : (W <= kMaxReg2W ? 2 : 1); }
+
+// Listed windows (all in order without idx), NW per thread; a window past the
+// list repeats its last and is not stored.  A group's samples are loaded one
+// group ahead.
+template <int W, bool EU, int NW>
+__global__ void __launch_bounds__(kRegBlock, 1)
 cdtw_reg_kernel(const float* __restrict__ x, const double* __restrict__ mu,
                 const float* __restrict__ sigma, const float4* __restrict__ qpad4, int lq4,
                 int M, int Nw, const int32_t* __restrict__ idx, int L, float* __restrict__ out) {
     extern __shared__ float4 sq4[];
-    for (int e = threadIdx.x; e < 4 * lq4; e += blockDim.x) sq4[e] = qpad4[e];
+    for (int e = threadIdx.x; e < lq4; e += blockDim.x) sq4[e] = qpad4[e];
     __syncthreads();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= L) return;
-    const int w = idx ? idx[t] : t;
-    if (w < 0 || w >= Nw) {  // a listed window outside the subject: NaN, no access
-        out[t] = __int_as_float(0x7fc00000);
-        return;
-    }
-    const Norm nm = make_norm(mu[w], sigma[w]);
-    const float* __restrict__ xw = x + w;
-
-    constexpr int B = 2 * W + 1;
-    constexpr int NQ4 = (B + 3) / 4;
-    float prev[B + 1];
-#pragma unroll
-    for (int k = 0; k <= B; ++k) prev[k] = CDTW_INF;
-    prev[W] = 0.0f;  // virtual D[-1][-1] = 0 (cdtw.cuh:35, :191)
-    float res = CDTW_INF;
-
-    for (int j0 = 0; j0 < M; j0 += 4) {
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int j = j0 + u;
-            const float z = znorm(nm, __ldg(xw + min(j, M - 1)));
-            const float4* qr = sq4 + u * lq4 + (j0 >> 2);
-            float qv[NQ4 * 4];
-#pragma unroll
-            for (int r = 0; r < NQ4; ++r) {
-                const float4 v = qr[r];
-                qv[4 * r + 0] = v.x;
-                qv[4 * r + 1] = v.y;
-                qv[4 * r + 2] = v.z;
-                qv[4 * r + 3] = v.w;
-            }
-            float left = CDTW_INF;
-            float cur[B];
-#pragma unroll
-            for (int k = 0; k < B; ++k) {
-                const float m = min3f(prev[k], prev[k + 1], left);
-                left = cell<EU>(z - qv[k], m);
-                cur[k] = left;
-            }
-            if (j == M - 1) res = cur[W];
-#pragma unroll
-            for (int k = 0; k < B; ++k) prev[k] = cur[k];
-        }
-    }
-    out[t] = res;
-}
-
-// Two windows per thread: both read the same query band values at a row (the
-// band of row j is q[j-W .. j+W] whatever the window), so the shared-memory
-// query loads are paid once for 2(2W+1) cells, and the two windows' cell
-// chains interleave (two independent min chains per thread).  Listed windows
-// 2t and 2t+1; a missing second window computes a copy of the first and is
-// not stored.
-constexpr int kMaxReg2W = 48;
-
-template <int W, bool EU>
-__global__ void __launch_bounds__(kRegBlock, 1)
-cdtw_reg2_kernel(const float* __restrict__ x, const double* __restrict__ mu,
-                 const float* __restrict__ sigma, const float4* __restrict__ qpad4, int lq4,
-                 int M, int Nw, const int32_t* __restrict__ idx, int L, float* __restrict__ out) {
-    extern __shared__ float4 sq4[];
-    for (int e = threadIdx.x; e < 4 * lq4; e += blockDim.x) sq4[e] = qpad4[e];
-    __syncthreads();
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (2 * t >= L) return;
-    const int t1 = min(2 * t + 1, L - 1);
-    int w0 = idx ? idx[2 * t] : 2 * t;
-    int w1 = idx ? idx[t1] : t1;
-    const bool ok0 = w0 >= 0 && w0 < Nw, ok1 = w1 >= 0 && w1 < Nw;
-    if (!ok0) w0 = 0;  // a listed window outside the subject: NaN, no access
-    if (!ok1) w1 = 0;
-    const Norm n0 = make_norm(mu[w0], sigma[w0]);
-    const Norm n1 = make_norm(mu[w1], sigma[w1]);
-    const float* __restrict__ x0 = x + w0;
-    const float* __restrict__ x1 = x + w1;
-
-    constexpr int B = 2 * W + 1;
-    constexpr int NQ4 = (B + 3) / 4;
-    float p0[B + 1], p1[B + 1];
-#pragma unroll
-    for (int k = 0; k <= B; ++k) {
-        p0[k] = CDTW_INF;
-        p1[k] = CDTW_INF;
-    }
-    p0[W] = 0.0f;
-    p1[W] = 0.0f;
-    float r0 = CDTW_INF, r1 = CDTW_INF;
-
-    for (int j0 = 0; j0 < M; j0 += 4) {
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int j = j0 + u;
-            const int jc = min(j, M - 1);
-            const float z0 = znorm(n0, __ldg(x0 + jc));
-            const float z1 = znorm(n1, __ldg(x1 + jc));
-            const float4* qr = sq4 + u * lq4 + (j0 >> 2);
-            float qv[NQ4 * 4];
-#pragma unroll
-            for (int r = 0; r < NQ4; ++r) {
-                const float4 v = qr[r];
-                qv[4 * r + 0] = v.x;
-                qv[4 * r + 1] = v.y;
-                qv[4 * r + 2] = v.z;
-                qv[4 * r + 3] = v.w;
-            }
-            float l0 = CDTW_INF, l1 = CDTW_INF;
-#pragma unroll
-            for (int k = 0; k < B; ++k) {
-                const float m0 = min3f(p0[k], p0[k + 1], l0);
-                const float m1 = min3f(p1[k], p1[k + 1], l1);
-                l0 = cell<EU>(z0 - qv[k], m0);
-                l1 = cell<EU>(z1 - qv[k], m1);
-                p0[k] = l0;  // p[k] is not read again this row
-                p1[k] = l1;
-            }
-            if (j == M - 1) {
-                r0 = p0[W];
-                r1 = p1[W];
-            }
-        }
-    }
-    out[2 * t] = ok0 ? r0 : __int_as_float(0x7fc00000);
-    if (2 * t + 1 < L) out[2 * t + 1] = ok1 ? r1 : __int_as_float(0x7fc00000);
-}
-
-// Four windows per thread for narrow bands: the query band values of a row
-// are loaded once for 4(2W+1) cells and four independent min chains
-// interleave (listed windows 4t .. 4t+3; missing ones repeat the last listed
-// window and are not stored).
-constexpr int kMaxReg4W = 16;
-
-template <int W, bool EU>
-__global__ void __launch_bounds__(kRegBlock, 1)
-cdtw_reg4_kernel(const float* __restrict__ x, const double* __restrict__ mu,
-                 const float* __restrict__ sigma, const float4* __restrict__ qpad4, int lq4,
-                 int M, int Nw, const int32_t* __restrict__ idx, int L, float* __restrict__ out) {
-    extern __shared__ float4 sq4[];
-    for (int e = threadIdx.x; e < 4 * lq4; e += blockDim.x) sq4[e] = qpad4[e];
-    __syncthreads();
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (4 * t >= L) return;
-    constexpr int NW = 4;
-    constexpr int B = 2 * W + 1;
-    constexpr int NQ4 = (B + 3) / 4;
+    if ((int64_t)NW * t >= L) return;
     Norm nm[NW];
     const float* xw[NW];
     bool ok[NW];
+    float xn[NW][4], res[NW];
 #pragma unroll
     for (int v = 0; v < NW; ++v) {
-        const int tv = min(4 * t + v, L - 1);
+        const int tv = min(NW * t + v, L - 1);
         int w = idx ? idx[tv] : tv;
         ok[v] = w >= 0 && w < Nw;
         if (!ok[v]) w = 0;  // a listed window outside the subject: NaN, no access
         nm[v] = make_norm(mu[w], sigma[w]);
         xw[v] = x + w;
+        res[v] = CDTW_INF;
+#pragma unroll
+        for (int r = 0; r < 4; ++r) xn[v][r] = __ldg(xw[v] + min(r, M - 1));
     }
-    float p[NW][B + 1];
-#pragma unroll
-    for (int v = 0; v < NW; ++v) {
-#pragma unroll
-        for (int k = 0; k <= B; ++k) p[v][k] = CDTW_INF;
-        p[v][W] = 0.0f;
-    }
-    float r[NW];
-#pragma unroll
-    for (int v = 0; v < NW; ++v) r[v] = CDTW_INF;
+    float p[NW][2 * W + 2];
+    reg_init<W, NW>(p);
     for (int j0 = 0; j0 < M; j0 += 4) {
+        float z[NW][4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int j = j0 + u;
-            const int jc = min(j, M - 1);
-            float z[NW];
+        for (int v = 0; v < NW; ++v) {
 #pragma unroll
-            for (int v = 0; v < NW; ++v) z[v] = znorm(nm[v], __ldg(xw[v] + jc));
-            const float4* qr = sq4 + u * lq4 + (j0 >> 2);
-            float qv[NQ4 * 4];
-#pragma unroll
-            for (int q4 = 0; q4 < NQ4; ++q4) {
-                const float4 a = qr[q4];
-                qv[4 * q4 + 0] = a.x;
-                qv[4 * q4 + 1] = a.y;
-                qv[4 * q4 + 2] = a.z;
-                qv[4 * q4 + 3] = a.w;
-            }
-            float l[NW];
-#pragma unroll
-            for (int v = 0; v < NW; ++v) l[v] = CDTW_INF;
-#pragma unroll
-            for (int k = 0; k < B; ++k) {
-#pragma unroll
-                for (int v = 0; v < NW; ++v) {
-                    const float m = min3f(p[v][k], p[v][k + 1], l[v]);
-                    l[v] = cell<EU>(z[v] - qv[k], m);
-                    p[v][k] = l[v];  // p[v][k] is not read again this row
-                }
-            }
-            if (j == M - 1) {
-#pragma unroll
-                for (int v = 0; v < NW; ++v) r[v] = p[v][W];
+            for (int r = 0; r < 4; ++r) {
+                z[v][r] = znorm(nm[v], xn[v][r]);
+                xn[v][r] = __ldg(xw[v] + min(j0 + 4 + r, M - 1));
             }
         }
+        reg_rows4<W, EU, NW, true>(p, z, sq4 + (j0 >> 2), M - 1 - j0, res);
     }
 #pragma unroll
     for (int v = 0; v < NW; ++v)
-        if (4 * t + v < L) out[4 * t + v] = ok[v] ? r[v] : __int_as_float(0x7fc00000);
+        if (NW * t + v < L) out[NW * t + v] = ok[v] ? res[v] : __int_as_float(0x7fc00000);
 }
 
 // All windows, NW consecutive ones per thread (windows NW t .. NW t + NW - 1,
 // no index list): window v's sample at row j is x[NW t + v + j], so the NW
-// windows of a thread read one sliding run of the stream.  Rows go in groups
-// of four; a group needs NW + 3 consecutive samples, of which four are new:
-// they are loaded one group ahead and the run is shifted by four at the end
-// of the group.  Every group but the last runs without row-index clamps or
-// result tests; the last (one to four rows) ends at row M - 1.
-template <int W, bool EU, int NW>
-__device__ __forceinline__ void regc_row(float (&p)[NW][2 * W + 2], const float (&z)[NW],
-                                         const float4* qr) {
-    constexpr int B = 2 * W + 1;
-    constexpr int NQ4 = (B + 3) / 4;
-    float qv[NQ4 * 4];
-#pragma unroll
-    for (int r = 0; r < NQ4; ++r) {
-        const float4 a = qr[r];
-        qv[4 * r + 0] = a.x;
-        qv[4 * r + 1] = a.y;
-        qv[4 * r + 2] = a.z;
-        qv[4 * r + 3] = a.w;
-    }
-    float l[NW];
-#pragma unroll
-    for (int v = 0; v < NW; ++v) l[v] = CDTW_INF;
-#pragma unroll
-    for (int k = 0; k < B; ++k) {
-#pragma unroll
-        for (int v = 0; v < NW; ++v) {
-            const float m = min3f(p[v][k], p[v][k + 1], l[v]);
-            l[v] = cell<EU>(z[v] - qv[k], m);
-            p[v][k] = l[v];  // p[v][k] is not read again this row
-        }
-    }
-}
-
+// windows of a thread read one sliding run of the stream.  A group of four
+// rows needs NW + 3 consecutive samples, of which four are new: they are
+// loaded one group ahead and the run is shifted by four at the end of the
+// group.  Every group but the last runs without result tests; the last (one to
+// four rows) ends at row M - 1.
 template <int W, bool EU, int NW>
 __global__ void __launch_bounds__(kRegBlock, 1)
 cdtw_regc_kernel(const float* __restrict__ x, const double* __restrict__ mu,
                  const float* __restrict__ sigma, const float4* __restrict__ qpad4, int lq4,
                  int M, int Nw, float* __restrict__ out) {
     extern __shared__ float4 sq4[];
-    for (int e = threadIdx.x; e < 4 * lq4; e += blockDim.x) sq4[e] = qpad4[e];
+    for (int e = threadIdx.x; e < lq4; e += blockDim.x) sq4[e] = qpad4[e];
     __syncthreads();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const int w0 = t * NW;
     if (w0 >= Nw) return;
-    constexpr int B = 2 * W + 1;
     constexpr int NX = NW + 3;  // samples of a group of four rows
     // the last thread's missing windows repeat window Nw - 1's statistics and
     // read clamped samples; they are not stored
@@ -305,95 +212,70 @@ cdtw_regc_kernel(const float* __restrict__ x, const double* __restrict__ mu,
         const int w = w0 + min(v, rem);
         nm[v] = make_norm(mu[w], sigma[w]);
     }
-    float p[NW][B + 1];
+    float p[NW][2 * W + 2], res[NW];
+    reg_init<W, NW>(p);
 #pragma unroll
-    for (int v = 0; v < NW; ++v) {
-#pragma unroll
-        for (int k = 0; k <= B; ++k) p[v][k] = CDTW_INF;
-        p[v][W] = 0.0f;
-    }
+    for (int v = 0; v < NW; ++v) res[v] = CDTW_INF;
     float xs[NX];
 #pragma unroll
     for (int i = 0; i < NX; ++i) xs[i] = __ldg(xb + min(i, xlast));
+    auto samples = [&](float (&z)[NW][4]) {
+#pragma unroll
+        for (int v = 0; v < NW; ++v) {
+#pragma unroll
+            for (int r = 0; r < 4; ++r) z[v][r] = znorm(nm[v], xs[r + v]);
+        }
+    };
     int j0 = 0;
     for (; j0 + 4 < M; j0 += 4) {
-        float nx[4];
+        float nx[4], z[NW][4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) nx[i] = __ldg(xb + min(j0 + NX + i, xlast));
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            float z[NW];
-#pragma unroll
-            for (int v = 0; v < NW; ++v) z[v] = znorm(nm[v], xs[u + v]);
-            regc_row<W, EU, NW>(p, z, sq4 + u * lq4 + (j0 >> 2));
-        }
+        samples(z);
+        reg_rows4<W, EU, NW, false>(p, z, sq4 + (j0 >> 2), 0, res);
 #pragma unroll
         for (int i = 0; i + 4 < NX; ++i) xs[i] = xs[i + 4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) xs[NX - 4 + i] = nx[i];
     }
-    float r[NW];
-#pragma unroll
-    for (int v = 0; v < NW; ++v) r[v] = CDTW_INF;
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-        if (j0 + u < M) {
-            float z[NW];
-#pragma unroll
-            for (int v = 0; v < NW; ++v) z[v] = znorm(nm[v], xs[u + v]);
-            regc_row<W, EU, NW>(p, z, sq4 + u * lq4 + (j0 >> 2));
-            if (j0 + u == M - 1) {
-#pragma unroll
-                for (int v = 0; v < NW; ++v) r[v] = p[v][W];
-            }
-        }
-    }
+    float z[NW][4];
+    samples(z);
+    reg_rows4<W, EU, NW, true>(p, z, sq4 + (j0 >> 2), M - 1 - j0, res);
 #pragma unroll
     for (int v = 0; v < NW; ++v)
-        if (v <= rem) out[w0 + v] = r[v];
+        if (v <= rem) out[w0 + v] = res[v];
 }
 
 using RegCKernel = void (*)(const float*, const double*, const float*, const float4*, int, int,
                             int, float*);
 
-// Windows per thread of the consecutive-window kernels (register budget: the
-// three-window kernel spills from W = 32).
-constexpr int kMaxReg3W = 31;
-constexpr int regc_per_thread(int W) {
-    return W <= kMaxReg4W ? 4 : (W <= kMaxReg3W ? 3 : 2);
-}
-
-template <int LO, int HI, int NW>
+template <int LO, int HI>
 struct RegCRange {
     static void fill(RegCKernel* eu, RegCKernel* mh) {
         if constexpr (LO <= HI) {
-            eu[LO] = cdtw_regc_kernel<LO, true, NW>;
-            mh[LO] = cdtw_regc_kernel<LO, false, NW>;
-            RegCRange<LO + 1, HI, NW>::fill(eu, mh);
+            eu[LO] = cdtw_regc_kernel<LO, true, reg_per_thread(LO)>;
+            mh[LO] = cdtw_regc_kernel<LO, false, reg_per_thread(LO)>;
+            RegCRange<LO + 1, HI>::fill(eu, mh);
         }
     }
 };
 
 // cDTW of one window (xw, normalisation nm) against the query whose padded
-// copies sit in shared memory (sq4, lq4 float4 per copy) with its envelope
-// senv, abandoning once the last row minimum plus the remaining suffix of the
-// window's forward LB_Keogh lbk (the cumulative bound cb of
-// UCR_DTW_BIN.cpp:666-677, :336) reaches the best-so-far in *key.  alive
-// marks lanes still worth finishing; the warp stops when no lane is.  All 32
-// lanes call together.  Returns +inf if the warp stopped early.
+// copy sits in shared memory (sq4) with its envelope senv, abandoning once the
+// last row minimum plus the remaining suffix of the window's forward LB_Keogh
+// lbk (the cumulative bound cb of UCR_DTW_BIN.cpp:666-677, :336) reaches the
+// best-so-far in *key.  alive marks lanes still worth finishing; the warp stops
+// when no lane is.  All 32 lanes call together.  Returns +inf if the warp
+// stopped early.
 template <int W, bool EU>
-__device__ __forceinline__ float reg_window_dtw(const float4* sq4, int lq4,
-                                                const float2* senv, int M,
+__device__ __forceinline__ float reg_window_dtw(const float4* sq4, const float2* senv, int M,
                                                 const float* __restrict__ xw, const Norm& nm,
                                                 float lbk, bool& alive,
                                                 const unsigned long long* key) {
     constexpr int B = 2 * W + 1;
-    constexpr int NQ4 = (B + 3) / 4;
-    float prev[B + 1];
-#pragma unroll
-    for (int k = 0; k <= B; ++k) prev[k] = CDTW_INF;
-    prev[W] = 0.0f;
-    float res = CDTW_INF, pre = 0.f;
+    float p[1][B + 1], z[1][4], res[1] = {CDTW_INF};
+    reg_init<W, 1>(p);
+    float pre = 0.f;
     // W <= 64: the samples of the next 4-row group are loaded one group ahead
     // (with few windows in flight their latency is not hidden by other warps;
     // wider bands leave no registers for it)
@@ -418,44 +300,23 @@ __device__ __forceinline__ float reg_window_dtw(const float4* sq4, int lq4,
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
             const int j = j0 + u;
-            const int jc = min(j, M - 1);
-            const float z = znorm(nm, xc[u]);
+            z[0][u] = znorm(nm, xc[u]);
             // forward LB_Keogh term of this data row (query envelope at j)
-            const float2 e = senv[jc];
-            const float dl = max3f(z - e.y, e.x - z, 0.f);
+            const float2 e = senv[min(j, M - 1)];
+            const float dl = max3f(z[0][u] - e.y, e.x - z[0][u], 0.f);
             pre += (j < M) ? (EU ? dl * dl : dl) : 0.f;
-            const float4* qr = sq4 + u * lq4 + (j0 >> 2);
-            float qv[NQ4 * 4];
-#pragma unroll
-            for (int r = 0; r < NQ4; ++r) {
-                const float4 v = qr[r];
-                qv[4 * r + 0] = v.x;
-                qv[4 * r + 1] = v.y;
-                qv[4 * r + 2] = v.z;
-                qv[4 * r + 3] = v.w;
-            }
-            float left = CDTW_INF;
-            float cur[B];
-#pragma unroll
-            for (int k = 0; k < B; ++k) {
-                const float m = min3f(prev[k], prev[k + 1], left);
-                left = cell<EU>(z - qv[k], m);
-                cur[k] = left;
-            }
-            if (j == M - 1) res = cur[W];
-#pragma unroll
-            for (int k = 0; k < B; ++k) prev[k] = cur[k];
         }
+        reg_rows4<W, EU, 1, true>(p, z, sq4 + (j0 >> 2), M - 1 - j0, res);
         if (check) {
-            float rmin = prev[0];
+            float rmin = p[0][0];
 #pragma unroll
-            for (int k = 1; k < B; k += 2) rmin = min3f(rmin, prev[k], prev[k + 1]);
+            for (int k = 1; k < B; k += 2) rmin = min3f(rmin, p[0][k], p[0][k + 1]);
             alive = alive && (rmin + lb_suffix(lbk, pre, M) * kLbSlack <
                               (kAhead ? bsf_early : load_bsf(key)));
             if (!__any_sync(0xffffffffu, alive)) return CDTW_INF;
         }
     }
-    return res;
+    return res[0];
 }
 
 // Search variant: persistent warps take 32 candidates at a time from a device
@@ -471,8 +332,8 @@ cdtw_reg_search_kernel(const float* __restrict__ x, const double* __restrict__ m
                        const int* __restrict__ count, int* __restrict__ work,
                        unsigned long long* __restrict__ key, const HitSink sink) {
     extern __shared__ float4 sq4[];
-    float2* senv = (float2*)(sq4 + 4 * lq4);
-    for (int e = threadIdx.x; e < 4 * lq4; e += blockDim.x) sq4[e] = qpad4[e];
+    float2* senv = (float2*)(sq4 + lq4);
+    for (int e = threadIdx.x; e < lq4; e += blockDim.x) sq4[e] = qpad4[e];
     for (int e = threadIdx.x; e < M; e += blockDim.x) senv[e] = qenv[e];
     __syncthreads();
     const int lane = threadIdx.x & 31;
@@ -491,7 +352,7 @@ cdtw_reg_search_kernel(const float* __restrict__ x, const double* __restrict__ m
         bool alive = (i < n) && (c.lb * kLbSlack < load_bsf(key));
         if (!__any_sync(0xffffffffu, alive)) continue;
         const Norm nm = make_norm(mu[c.w], sigma[c.w]);
-        const float res = reg_window_dtw<W, EU>(sq4, lq4, senv, M, x + c.w, nm, c.lbk, alive, key);
+        const float res = reg_window_dtw<W, EU>(sq4, senv, M, x + c.w, nm, c.lbk, alive, key);
         if (i < n && res < CDTW_INF) report_window(key, sink, res, (uint32_t)c.w);
     }
 }
@@ -502,13 +363,14 @@ using RegSearchKernel = void (*)(const float*, const double*, const float*, cons
                                  const float2*, int, const Cand*, const int*, int*,
                                  unsigned long long*, const HitSink);
 
-// Instantiates the kernels for bands LO..HI into the dispatch tables.
+// Instantiates the one-window and the search kernels for bands LO..HI into the
+// dispatch tables.
 template <int LO, int HI>
 struct RegRange {
     static void fill(RegKernel* eu, RegKernel* mh, RegSearchKernel* seu, RegSearchKernel* smh) {
         if constexpr (LO <= HI) {
-            eu[LO] = cdtw_reg_kernel<LO, true>;
-            mh[LO] = cdtw_reg_kernel<LO, false>;
+            eu[LO] = cdtw_reg_kernel<LO, true, 1>;
+            mh[LO] = cdtw_reg_kernel<LO, false, 1>;
             seu[LO] = cdtw_reg_search_kernel<LO, true>;
             smh[LO] = cdtw_reg_search_kernel<LO, false>;
             RegRange<LO + 1, HI>::fill(eu, mh, seu, smh);
@@ -516,29 +378,19 @@ struct RegRange {
     }
 };
 
+// Several windows per thread, where the band leaves the registers for it.
+template <int LO, int HI>
+struct RegNRange {
+    static void fill(RegKernel* eu, RegKernel* mh) {
+        if constexpr (LO <= HI) {
+            eu[LO] = cdtw_reg_kernel<LO, true, reg_per_thread(LO)>;
+            mh[LO] = cdtw_reg_kernel<LO, false, reg_per_thread(LO)>;
+            RegNRange<LO + 1, HI>::fill(eu, mh);
+        }
+    }
+};
+
 }  // namespace
-
-template <int LO, int HI>
-struct Reg2Range {
-    static void fill(RegKernel* eu, RegKernel* mh) {
-        if constexpr (LO <= HI) {
-            eu[LO] = cdtw_reg2_kernel<LO, true>;
-            mh[LO] = cdtw_reg2_kernel<LO, false>;
-            Reg2Range<LO + 1, HI>::fill(eu, mh);
-        }
-    }
-};
-
-template <int LO, int HI>
-struct Reg4Range {
-    static void fill(RegKernel* eu, RegKernel* mh) {
-        if constexpr (LO <= HI) {
-            eu[LO] = cdtw_reg4_kernel<LO, true>;
-            mh[LO] = cdtw_reg4_kernel<LO, false>;
-            Reg4Range<LO + 1, HI>::fill(eu, mh);
-        }
-    }
-};
 
 // Defined in cdtw_reg_part*.cu: each fills its range of bands.
 void reg_fill_part0(void** eu, void** mh, void** seu, void** smh);
@@ -547,13 +399,12 @@ void reg_fill_part2(void** eu, void** mh, void** seu, void** smh);
 void reg_fill_part3(void** eu, void** mh, void** seu, void** smh);
 void reg_fill_part4(void** eu, void** mh, void** seu, void** smh);
 void reg_fill_part5(void** eu, void** mh, void** seu, void** smh);
-void reg2_fill_part0(void** eu, void** mh);  // two-window kernels, cdtw_reg2_part*.cu
-void reg2_fill_part1(void** eu, void** mh);
-void reg4_fill_part0(void** eu, void** mh);  // four-window kernels, cdtw_reg4_part0.cu
-// all-windows kernels over consecutive windows (cdtw_regc_part*.cu), windows
-// per thread regc_per_thread(W)
+void regn_fill_part0(void** eu, void** mh);  // several windows, cdtw_regn_part0.cu
+// all-windows kernels over consecutive windows (cdtw_regc_part*.cu)
 void regc_fill_part0(void** eu, void** mh);
 void regc_fill_part1(void** eu, void** mh);
 void regc_fill_part2(void** eu, void** mh);
+void regc_fill_part3(void** eu, void** mh);
+void regc_fill_part4(void** eu, void** mh);
 
 }  // namespace cdtw

@@ -1,4 +1,4 @@
-// All-windows register-band cDTW over consecutive windows, four windows per thread, W = 0..16
+// All-windows register-band cDTW over consecutive windows
 // (see cdtw_reg.cuh); one translation unit per band range for a parallel
 // build.
 #include "cdtw_reg.cuh"
@@ -6,7 +6,7 @@
 namespace cdtw {
 
 void regc_fill_part0(void** eu, void** mh) {
-    RegCRange<0, kMaxReg4W, 4>::fill((RegCKernel*)eu, (RegCKernel*)mh);
+    RegCRange<0, 24>::fill((RegCKernel*)eu, (RegCKernel*)mh);
 }
 
 }  // namespace cdtw
