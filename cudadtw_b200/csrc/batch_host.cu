@@ -302,10 +302,10 @@ extern "C" int cdtw_search_batched(cdtw_handle h, const float* d_subject, int64_
         if (Ws[q] < 0) return set_error(h, CDTW_EINVAL, "query %d: negative band", q);
         W[q] = std::min(Ws[q], M[q] - 1);
         // 0 = register-band main pass (W <= 96), else strip rows
-        R[q] = rows ? rows[q] : (W[q] <= max_register_band() ? 0 : 16);
+        R[q] = rows ? rows[q] : (W[q] <= max_batch_register_band() ? 0 : 16);
         if (R[q] != 0 && R[q] != 1 && R[q] != 2 && R[q] != 4 && R[q] != 8 && R[q] != 16)
             return set_error(h, CDTW_EINVAL, "query %d: rows must be 0, 1, 2, 4, 8 or 16", q);
-        if (R[q] == 0 && W[q] > max_register_band()) R[q] = 16;
+        if (R[q] == 0 && W[q] > max_batch_register_band()) R[q] = 16;
         if (R[q] > W[q] + 1) R[q] = default_rows(W[q]);
         T[q] = tiles ? tiles[q] : 1024;
         if (T[q] < 32 || T[q] > 4096 || (T[q] & 31))

@@ -9,8 +9,8 @@ namespace cdtw {
 namespace {
 
 struct BatchRegKernels {
-    BatchRegKernel eu[kMaxRegW + 1];
-    BatchRegKernel mh[kMaxRegW + 1];
+    BatchRegKernel eu[kMaxBatchRegW + 1];
+    BatchRegKernel mh[kMaxBatchRegW + 1];
     BatchRegKernels() {
         void** a = (void**)eu;
         void** b = (void**)mh;
@@ -31,7 +31,7 @@ const BatchRegKernels& batch_reg_kernels() {
 }  // namespace
 
 int batch_reg_prepare(cdtw_handle h, int W, bool euclid, size_t smem, int* blocks) {
-    if (W < 0 || W > kMaxRegW) return set_error(h, CDTW_EINVAL, "register band %d out of range", W);
+    if (W < 0 || W > kMaxBatchRegW) return set_error(h, CDTW_EINVAL, "register band %d out of range", W);
     const void* k = (const void*)(euclid ? batch_reg_kernels().eu[W] : batch_reg_kernels().mh[W]);
     if (smem > 48 * 1024)
         CDTW_CUDA(h, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -49,5 +49,7 @@ int launch_batch_reg(cdtw_handle h, const BatchArgs& b, int W, bool euclid, size
     CDTW_LAUNCH(h, "batch_reg_kernel");
     return CDTW_OK;
 }
+
+int max_batch_register_band() { return kMaxBatchRegW; }
 
 }  // namespace cdtw

@@ -50,6 +50,8 @@ batch_reg_kernel(const BatchArgs b) {
     }
 }
 
+constexpr int kMaxBatchRegW = 96;  // instantiated bands 0..kMaxBatchRegW
+
 using BatchRegKernel = void (*)(const BatchArgs);
 
 template <int LO, int HI>

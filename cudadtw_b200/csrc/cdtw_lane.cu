@@ -130,6 +130,7 @@ int fill_lane_args(cdtw_handle h, const float* x, int64_t N, const double* mu,
     a->cands = nullptr;
     a->count = nullptr;
     a->work = nullptr;
+    a->nsm = h->sm_count;
     a->key = nullptr;
     return CDTW_OK;
 }
@@ -197,6 +198,7 @@ int launch_cdtw_lane_search(cdtw_handle h, const float* x, int64_t N, const doub
     a.cands = cands;
     a.count = count;
     a.work = work;
+    a.nsm = h->sm_count;
     a.key = key;
     a.sink = sink;
     const LaneKernel k = euclid ? lane_kernels().seu[B] : lane_kernels().smh[B];

@@ -62,6 +62,7 @@ struct LaneArgs {
     const Cand* cands;
     const int* count;
     int* work;
+    int nsm;  // SMs of the device
     unsigned long long* key;
     HitSink sink;
 };
@@ -353,11 +354,8 @@ cdtw_lane_search_kernel(const LaneArgs a) {
     const int h = lane >> a.lgG;  // group in warp
     const int per_warp = 64 >> a.lgG;
     const int n = *(const volatile int*)a.count;
-    for (;;) {
-        int base = 0;
-        if (lane == 0) base = atomicAdd(a.work, per_warp);
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (base >= n) break;
+    for (int base = first_batch(a.work, per_warp, a.nsm); base < n;
+         base = next_batch(a.work, per_warp)) {
         const int i0 = base + 2 * h, i1 = base + 2 * h + 1;
         Cand c0, c1;
         c0.w = 0;

@@ -26,12 +26,15 @@ struct RegKernels {
         reg_fill_part3(a, b, c, d);
         reg_fill_part4(a, b, c, d);
         reg_fill_part5(a, b, c, d);
+        reg_fill_part6(a, b, c, d);
+        reg_fill_part7(a, b, c, d);
         regn_fill_part0((void**)eun, (void**)mhn);
         regc_fill_part0((void**)euc, (void**)mhc);
         regc_fill_part1((void**)euc, (void**)mhc);
         regc_fill_part2((void**)euc, (void**)mhc);
         regc_fill_part3((void**)euc, (void**)mhc);
         regc_fill_part4((void**)euc, (void**)mhc);
+        regc_fill_part5((void**)euc, (void**)mhc);
     }
 };
 
@@ -41,8 +44,6 @@ const RegKernels& reg_kernels() {
 }
 
 }  // namespace
-
-int max_register_band() { return kMaxRegW; }
 
 int choose_variant(cdtw_handle h, int W) {
     int v = (W >= 0 && W < CDTW_MAX_QUERY) ? h->band_variant[W] : 0;
@@ -58,6 +59,22 @@ int choose_variant(cdtw_handle h, int W) {
     return v;
 }
 
+// The search's kernel: bands above kLaneSearchW over few windows keep the lane
+// groups, whose windows take a quarter of a thread's time each (M = 1000,
+// W = 100: 32k windows 1.06 ms on the register band and 1.00 on lane groups,
+// 262k 2.8 and 4.1).
+int search_variant(cdtw_handle h, int W, int64_t Nw) {
+    constexpr int kLaneSearchW = 96;
+    constexpr int64_t kLaneSearchWindows = 1 << 16;
+    const int v = choose_variant(h, W);
+    int G, B;
+    if (v == CDTW_VARIANT_REGISTER && W > kLaneSearchW && Nw < kLaneSearchWindows &&
+        h->band_variant[W] == CDTW_VARIANT_AUTO && lane_shape(W, &G, &B) &&
+        h->q.lq >= lane_qpad_min(h->q.M, W))
+        return CDTW_VARIANT_LANE;
+    return v;
+}
+
 int launch_cdtw_strip_search(cdtw_handle h, const float* x, int64_t N, const double* mu,
                              const float* sigma, const Cand* cands, const int* count, int* work,
                              int max_count, bool euclid, int R, unsigned long long* key,
@@ -69,7 +86,7 @@ int launch_cdtw_search(cdtw_handle h, const float* x, int64_t N, const double* m
                        const HitSink& sink) {
     const QueryPack& q = h->q;
     if (max_count <= 0) return CDTW_OK;
-    const int variant = choose_variant(h, q.W);
+    const int variant = search_variant(h, q.W, N - q.M + 1);
     if (variant == CDTW_VARIANT_LANE)
         return launch_cdtw_lane_search(h, x, N, mu, sigma, cands, count, work, max_count, euclid,
                                        key, sink);
@@ -89,7 +106,7 @@ int launch_cdtw_search(cdtw_handle h, const float* x, int64_t N, const double* m
     const unsigned blocks = (unsigned)std::max<int64_t>(
         1, std::min<int64_t>(want, (int64_t)std::max(per_sm, 1) * h->sm_count));
     k<<<blocks, kRegBlock, smem, h->stream>>>(x, mu, sigma, (const float4*)q.qpad, lq4, q.env,
-                                              q.M, cands, count, work, key, sink);
+                                              q.M, cands, count, work, key, sink, h->sm_count);
     CDTW_LAUNCH(h, "cdtw_reg_search_kernel");
     return CDTW_OK;
 }

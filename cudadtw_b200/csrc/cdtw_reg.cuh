@@ -44,7 +44,7 @@ namespace cdtw {
 namespace {
 
 constexpr int kRegBlock = 128;
-constexpr int kMaxRegW = 96;
+constexpr int kMaxRegW = 106;  // the widest band that 255 registers hold without spills
 
 // (x, y) as a packed FP32 pair, and the two differences of two pairs.
 __device__ __forceinline__ unsigned long long pack2(float x, float y) {
@@ -330,7 +330,7 @@ cdtw_reg_search_kernel(const float* __restrict__ x, const double* __restrict__ m
                        const float* __restrict__ sigma, const float4* __restrict__ qpad4, int lq4,
                        const float2* __restrict__ qenv, int M, const Cand* __restrict__ cands,
                        const int* __restrict__ count, int* __restrict__ work,
-                       unsigned long long* __restrict__ key, const HitSink sink) {
+                       unsigned long long* __restrict__ key, const HitSink sink, int nsm) {
     extern __shared__ float4 sq4[];
     float2* senv = (float2*)(sq4 + lq4);
     for (int e = threadIdx.x; e < lq4; e += blockDim.x) sq4[e] = qpad4[e];
@@ -338,11 +338,7 @@ cdtw_reg_search_kernel(const float* __restrict__ x, const double* __restrict__ m
     __syncthreads();
     const int lane = threadIdx.x & 31;
     const int n = *(const volatile int*)count;
-    for (;;) {
-        int base = 0;
-        if (lane == 0) base = atomicAdd(work, 32);
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (base >= n) break;
+    for (int base = first_batch(work, 32, nsm); base < n; base = next_batch(work, 32)) {
         const int i = base + lane;
         Cand c;
         c.w = 0;
@@ -361,7 +357,7 @@ using RegKernel = void (*)(const float*, const double*, const float*, const floa
                            int, const int32_t*, int, float*);
 using RegSearchKernel = void (*)(const float*, const double*, const float*, const float4*, int,
                                  const float2*, int, const Cand*, const int*, int*,
-                                 unsigned long long*, const HitSink);
+                                 unsigned long long*, const HitSink, int);
 
 // Instantiates the one-window and the search kernels for bands LO..HI into the
 // dispatch tables.
@@ -399,6 +395,8 @@ void reg_fill_part2(void** eu, void** mh, void** seu, void** smh);
 void reg_fill_part3(void** eu, void** mh, void** seu, void** smh);
 void reg_fill_part4(void** eu, void** mh, void** seu, void** smh);
 void reg_fill_part5(void** eu, void** mh, void** seu, void** smh);
+void reg_fill_part6(void** eu, void** mh, void** seu, void** smh);
+void reg_fill_part7(void** eu, void** mh, void** seu, void** smh);
 void regn_fill_part0(void** eu, void** mh);  // several windows, cdtw_regn_part0.cu
 // all-windows kernels over consecutive windows (cdtw_regc_part*.cu)
 void regc_fill_part0(void** eu, void** mh);
@@ -406,5 +404,6 @@ void regc_fill_part1(void** eu, void** mh);
 void regc_fill_part2(void** eu, void** mh);
 void regc_fill_part3(void** eu, void** mh);
 void regc_fill_part4(void** eu, void** mh);
+void regc_fill_part5(void** eu, void** mh);
 
 }  // namespace cdtw

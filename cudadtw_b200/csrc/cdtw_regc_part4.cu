@@ -6,7 +6,7 @@
 namespace cdtw {
 
 void regc_fill_part4(void** eu, void** mh) {
-    RegCRange<83, kMaxRegW>::fill((RegCKernel*)eu, (RegCKernel*)mh);
+    RegCRange<83, 96>::fill((RegCKernel*)eu, (RegCKernel*)mh);
 }
 
 }  // namespace cdtw

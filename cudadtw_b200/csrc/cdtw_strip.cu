@@ -40,15 +40,11 @@ __global__ void __launch_bounds__(kStripWarps * 32)
 cdtw_strip_search_kernel(const StripArgs a, const float2* __restrict__ qenv,
                          const Cand* __restrict__ cands, const int* __restrict__ count,
                          int* __restrict__ work, unsigned long long* __restrict__ key,
-                         const HitSink sink) {
+                         const HitSink sink, int nsm) {
     float* ring = lane_ring(a);
     const int lane = threadIdx.x & 31;
     const int n = *(const volatile int*)count;
-    for (;;) {
-        int base = 0;
-        if (lane == 0) base = atomicAdd(work, 32);
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (base >= n) break;
+    for (int base = first_batch(work, 32, nsm); base < n; base = next_batch(work, 32)) {
         const int i = base + lane;
         Cand c;
         c.w = 0;
@@ -138,7 +134,7 @@ int launch_cdtw_strip_search(cdtw_handle h, const float* x, int64_t N, const dou
         return set_error(h, CDTW_EUNSUPPORTED, "strip kernel needs W >= R-1 (W=%d R=%d)", q.W, R);
     if (max_count <= 0) return CDTW_OK;
     using SK = void (*)(const StripArgs, const float2*, const Cand*, const int*, int*,
-                        unsigned long long*, const HitSink);
+                        unsigned long long*, const HitSink, int);
     SK k;
     if (R == 16)
         k = euclid ? cdtw_strip_search_kernel<16, true> : cdtw_strip_search_kernel<16, false>;
@@ -150,7 +146,7 @@ int launch_cdtw_strip_search(cdtw_handle h, const float* x, int64_t N, const dou
     a.idx = nullptr;
     a.L = 0;
     a.out = nullptr;
-    k<<<blocks, kStripWarps * 32, 0, h->stream>>>(a, q.env, cands, count, work, key, sink);
+    k<<<blocks, kStripWarps * 32, 0, h->stream>>>(a, q.env, cands, count, work, key, sink, h->sm_count);
     CDTW_LAUNCH(h, "cdtw_strip_search_kernel");
     return CDTW_OK;
 }

@@ -332,6 +332,28 @@ __device__ __forceinline__ float load_bsf(const unsigned long long* key) {
     return (k == ~0ull) ? CDTW_INF : d;
 }
 
+// Work distribution of the search kernels' persistent warps: `step` candidates
+// a time from *work on.  The first round is dealt out by position, one batch a
+// block before any block gets a second (blocks go round the SMs, and the warp
+// that takes a block's first batch rotates with the block's layer, so a short
+// list lies on all SMs and schedulers: drawn from a counter, the 736 batches of
+// a 24k-candidate list went to the 26 SMs whose 28 warps started first, 57 us
+// against 18 on average over the SMs); later rounds come from a counter at
+// work[kWorkNext].  *work itself (the first candidate) is only read.
+constexpr int kWorkNext = 4;
+__device__ __forceinline__ int first_batch(const int* work, int step, int nsm) {
+    const int wpb = blockDim.x >> 5, wid = threadIdx.x >> 5;
+    const int turn = (wid + (int)blockIdx.x / nsm) % wpb;
+    return *work + (turn * (int)gridDim.x + (int)blockIdx.x) * step;
+}
+// All lanes of a warp call; step candidates from the returned index.
+__device__ __forceinline__ int next_batch(int* work, int step) {
+    int at = 0;
+    if ((threadIdx.x & 31) == 0) at = atomicAdd(work + kWorkNext, step);
+    at = __shfl_sync(0xffffffffu, at, 0);
+    return *work + (int)(gridDim.x * (blockDim.x >> 5)) * step + at;
+}
+
 // Where a search kernel puts a finished window: without a hit list, the
 // packed (distance, window) atomicMin into *key (argmin search); with one,
 // every window whose packed key is below *key is appended to the list (the
@@ -405,11 +427,13 @@ int launch_cdtw_lane_search(cdtw_handle h, const float* x, int64_t N, const doub
 // floats per shifted query copy (QueryPack::lq) of a handle's query pack
 inline int qpad_len(int M, int W) { return (int)(((int64_t)M + 2 * W + 56 + 3) / 4 * 4); }
 // Kernel choice for band W: CDTW_VARIANT_REGISTER (one thread per window, band
-// in registers, W <= 96), CDTW_VARIANT_STRIP16 / STRIP32 (strips of 16 / 32
+// in registers, W <= 106), CDTW_VARIANT_STRIP16 / STRIP32 (strips of 16 / 32
 // rows, W >= 15 / 31), CDTW_VARIANT_LANE (band over a lane group, 27 <= W <=
 // 767).
 int choose_variant(cdtw_handle h, int W);
-int max_register_band();
+// The search kernels' variant for band W over Nw windows.
+int search_variant(cdtw_handle h, int W, int64_t Nw);
+int max_batch_register_band();  // of the batched tile kernels
 int launch_lb_kim(cdtw_handle h, const float* x, int64_t N, const double* mu, const float* sigma,
                   const int32_t* idx, int64_t L, bool euclid, float* out,
                   unsigned long long* seeds = nullptr, unsigned* bmax = nullptr);
@@ -429,7 +453,8 @@ int launch_lb_keogh(cdtw_handle h, const float* x, int64_t N, const double* mu,
 // DTW over a device candidate list with early abandoning and a fused argmin
 // into *key (packed distance/index), or, with a hit list, the collection of
 // the windows below the threshold in *key.  `count` and `work` are device
-// ints.
+// ints: the candidates' number, the first one to take, and at
+// work[kWorkNext] a zero.
 int launch_cdtw_search(cdtw_handle h, const float* x, int64_t N, const double* mu,
                        const float* sigma, const Cand* cands, const int* count, int* work,
                        int max_count, bool euclid, unsigned long long* key,

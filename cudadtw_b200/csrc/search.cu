@@ -21,7 +21,7 @@
 //      and a thread per window (the count is read on the device).
 //   5. cDTW of the survivors with early abandoning against the live
 //      best-so-far, folded into the key: as pairwise wavefronts when few and
-//      long, else by the register-band (W <= 96) or lane-group kernels.
+//      long, else by the register-band (W <= 106) or lane-group kernels.
 // No sort, no host loop; graph-capturable launch sequence.
 #include "common.cuh"
 
@@ -42,7 +42,9 @@ struct SearchWs {
     Cand* q2 = nullptr;
     float2* xenv = nullptr;
     float* envscratch = nullptr;
-    // [0] n1, [1] n2, [2] work seeds, [3] work main, [4] n seeds, [5] largest LB_Kim (bits)
+    // [0] n1, [1] n2, [2] work seeds, [3] work main, [4] n seeds, [5] largest
+    // LB_Kim (bits), [6] and [7] (work + kWorkNext) the seeds' and the main
+    // pass's next batches
     int* ctr = nullptr;
     unsigned long long* key = nullptr;
     float* seed_z = nullptr;  // z-normalised seed windows (seed_cap floats)
@@ -76,7 +78,7 @@ __global__ void seed_gather_kernel(const float* __restrict__ x, const double* __
 // The survivors of the bounds when there are at most `cap`, z-normalised
 // exactly as the search kernels do (make_norm / znorm), for their pairwise
 // wavefront cDTW (which runs the first *count rows only).  Thread 0 starts
-// the search kernels' work counter at cap (they then find nothing left), or
+// the search kernels' candidates at cap (they then find nothing left), or
 // at 0 when there are more survivors than cap (the wavefront pass is skipped
 // and they take all).
 __global__ void wave_gather_kernel(const float* __restrict__ x, const double* __restrict__ mu,
@@ -970,7 +972,7 @@ int run_search(cdtw_handle h, const float* x, int64_t N, const double* mu, const
     //    the wavefronts: measured at M=1024, W=204, the wavefronts of 4373
     //    survivors took 0.53 ms.
     int wcap = (int)std::min<int64_t>(kWaveSurvivors, ws.seed_cap / q.M);
-    if (choose_variant(h, q.W) == CDTW_VARIANT_LANE) wcap = std::min(wcap, kWaveFew);
+    if (search_variant(h, q.W, Nw) == CDTW_VARIANT_LANE) wcap = std::min(wcap, kWaveFew);
     if (wave_eligible(q.M, q.W) && wcap >= 32) {
         wave_gather_kernel<<<(unsigned)div_up((int64_t)wcap * 32, 256), 256, 0, h->stream>>>(
             x, mu, sigma, ws.q2, ws.ctr + 1, wcap, q.M, ws.seed_z, ws.ctr + 3);

@@ -429,9 +429,9 @@ int cdtw_refine_templates_search(cdtw_handle h, const float* d_subject, int64_t 
 /* ---- kernel selection ----------------------------------------------------------- */
 
 enum cdtw_variant {
-    CDTW_VARIANT_AUTO = 0,      /* built-in rule: register band for W <= 96, lane groups up
+    CDTW_VARIANT_AUTO = 0,      /* built-in rule: register band for W <= 106, lane groups up
                                    to W = 767, 16-row strips above                      */
-    CDTW_VARIANT_REGISTER = 1,  /* one thread per window, the band in registers (W <= 96) */
+    CDTW_VARIANT_REGISTER = 1,  /* one thread per window, the band in registers (W <= 106) */
     CDTW_VARIANT_STRIP16 = 2,   /* strips of 16 rows, boundary ring (W >= 15)            */
     CDTW_VARIANT_STRIP32 = 3,   /* strips of 32 rows, boundary ring (W >= 31)            */
     CDTW_VARIANT_LANE = 4       /* band spread over a lane group, two windows per group
