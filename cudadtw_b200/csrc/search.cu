@@ -208,7 +208,19 @@ compact_kim_kernel(const float* __restrict__ lbkim, int Nw, const unsigned long 
     }
 }
 
-// Forward + reverse LB_Keogh of the compacted windows; survivors -> q2.
+__device__ __forceinline__ float warp_sum_f(float v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+// Forward + reverse LB_Keogh of the compacted windows against the stream's
+// envelope; survivors -> q2.  Up to kFilterWarps windows, where threads alone
+// would leave SMs without a block, a warp takes one (its loads coalesced, all
+// schedulers busy: searches with 29k LB_Kim survivors, M = 1000, W = 50, 523 ->
+// 456 us; with 125k, M = 128, 134 -> 173), above that a thread.
+constexpr int kFilterWarps = 1 << 15;
+
 template <bool EU>
 __global__ void __launch_bounds__(256)
 keogh_filter_kernel(const float* __restrict__ x, const double* __restrict__ mu,
@@ -222,6 +234,67 @@ keogh_filter_kernel(const float* __restrict__ x, const double* __restrict__ mu,
     const float bsf = load_bsf(key);
     const float lim = bsf / kLbSlack;  // bound value at which a window is pruned
     const int lane = threadIdx.x & 31;
+    if (n1 <= kFilterWarps) {
+        // a warp per window, lanes over its samples; both bounds abandoned
+        // every 128.  A warp takes neighbouring entries and appends their
+        // survivors together (lane c keeps the c-th): the search kernels' warps
+        // want neighbouring windows.
+        const int nwarps = (int)(gridDim.x * blockDim.x) >> 5;
+        const int per = min(32, (n1 + nwarps - 1) / nwarps);
+        const int first = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * per;
+        for (int i0 = first; i0 < n1; i0 += nwarps * per) {
+            int kept = 0;
+            Cand mine;
+            for (int i = i0; i < min(i0 + per, n1); ++i) {
+                const int w = q1[i];
+                const Norm nm = make_norm(mu[w], sigma[w]);
+                float af = 0.f, ar = 0.f, tf = 0.f, tr = 0.f;
+                bool pruned = false;
+                for (int k0 = 0; k0 < M && !pruned; k0 += 128) {
+                    float xv[4], qv[4];
+                    float2 ev[4], dv[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        const int k = min(k0 + 32 * u + lane, M - 1);
+                        xv[u] = __ldg(x + w + k);
+                        qv[u] = __ldg(zq + k);
+                        ev[u] = __ldg(qenv + k);
+                        dv[u] = __ldg(xenv + w + k);
+                    }
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        if (k0 + 32 * u + lane < M) {
+                            const float z = znorm(nm, xv[u]);
+                            const float df = max3f(z - ev[u].y, ev[u].x - z, 0.f);
+                            af = EU ? fmaf(df, df, af) : af + df;
+                            const float dr = max3f(qv[u] - znorm(nm, dv[u].y),
+                                                   znorm(nm, dv[u].x) - qv[u], 0.f);
+                            ar = EU ? fmaf(dr, dr, ar) : ar + dr;
+                        }
+                    }
+                    tf = warp_sum_f(af);
+                    tr = warp_sum_f(ar);
+                    pruned = fmaxf(tf, tr) >= lim;
+                }
+                const float lb = fmaxf(lbkim[w], fmaxf(tf, tr));
+                if (!pruned && lb < lim) {  // warp-uniform
+                    if (lane == kept) {
+                        mine.w = w;
+                        mine.lb = lb;
+                        mine.lbk = tf;
+                    }
+                    ++kept;
+                }
+            }
+            if (kept) {
+                int at = 0;
+                if (lane == 0) at = atomicAdd(n2, kept);
+                at = __shfl_sync(0xffffffffu, at, 0);
+                if (lane < kept) q2[at + lane] = mine;
+            }
+        }
+        return;
+    }
     for (int base = (blockIdx.x * blockDim.x + threadIdx.x) & ~31; base < n1;
          base += gridDim.x * blockDim.x) {
         const int i = base + lane;
@@ -266,12 +339,6 @@ keogh_filter_kernel(const float* __restrict__ x, const double* __restrict__ mu,
             q2[at + __popc(m & ((1u << lane) - 1))] = c;
         }
     }
-}
-
-__device__ __forceinline__ float warp_sum_f(float v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
 }
 
 constexpr int kSparseMaxWarps = 16;  // warps per block of keogh_sparse_kernel (at most)
@@ -520,10 +587,23 @@ keogh_sparse_kernel(const float* __restrict__ x, int64_t N, const double* __rest
 
 constexpr int kSparseSpanMax = 6144;  // M + 2W of the per-window envelope (96 KB a warp)
 constexpr int kSparseVHMinBand = 301;  // 2W+1 from which the van Herk blocks serve it
-// The dense regime (stream envelope + a thread per survivor) was also tried
-// from a per-window work estimate (span x doubling passes): at M=1024, W=102
-// and 204 it measured no faster than the per-window envelopes (586 against
-// 548 us; 1.17 against 0.83 ms per search), so the choice stays by count.
+// Survivors up to which a warp per window with its own envelope is the faster
+// way.  The stream envelope costs 7.1 ps a sample of the stream; a survivor
+// costs about 0.25 ns plus 0.35 ps per span sample and doubling pass with its
+// own envelope (van Herk counted as twelve passes), against 1.7 ps per sample
+// with the stream's.  2^25 samples, 250k to 425k survivors, search with the
+// stream envelope / own envelopes (us): M = 300, W = 15 678 / 531, W = 60
+// 856 / 815; M = 512, W = 25 806 / 632, W = 51 836 / 850, W = 102 1132 / 1512;
+// M = 1000, W = 50 1012 / 800, W = 100 1021 / 1269.
+int sparse_limit(int64_t N, int M, int W) {
+    const double span = M + 2.0 * W;
+    double passes = 1.0;
+    for (int p = 1; 2 * p <= 2 * W + 1; p *= 2) passes += 1.0;
+    if (2 * W + 1 >= kSparseVHMinBand) passes = 12.0;
+    const double own = 0.25 + 0.35e-3 * span * passes, shared = 1.7e-3 * M;
+    const double cut = own > shared ? 7.1e-3 * (double)N / (own - shared) : 1e9;
+    return (int)std::min(std::max(cut, (double)(N / 256)), (double)((int64_t)1 << 20));
+}
 
 // Forward + reverse LB_Keogh of the LB_Kim survivors q1 (count *n1, known
 // only on the device) into q2 / *n2: up to sparse_max survivors a warp per
@@ -537,8 +617,7 @@ int launch_keogh(cdtw_handle h, const float* x, int64_t N, const double* mu, con
     const int M = q.M, W = q.W;
     const int span = M + 2 * W;
     const int S = (int)round_up(span, 4);
-    const int sparse_max =
-        span <= kSparseSpanMax ? (int)std::min<int64_t>(N / 256, (int64_t)1 << 18) : -1;
+    const int sparse_max = span <= kSparseSpanMax ? sparse_limit(N, M, W) : -1;
     CDTW_TRY(launch_stream_envelope(h, x, N, W, ws.envscratch, ws.xenv, ws.ctr + 0, sparse_max));
     const int grid = h->sm_count * 8;
     if (euclid)
