@@ -425,36 +425,8 @@ int cdtw_topk(cdtw_handle h, const float* d_subject, int64_t N, const double* d_
         return set_error(h, CDTW_EINVAL, "subject length %lld for M=%d", (long long)N, M);
     if (M < 11) return set_error(h, CDTW_EUNSUPPORTED, "top-k search needs M >= 11");
     if (!valid_metric(metric)) return set_error(h, CDTW_EINVAL, "bad metric %d", metric);
-    CDTW_CUDA(h, cudaSetDevice(h->device));
-    CDTW_TRY(ensure_workspace(h, topk_workspace_bytes(N, M, h->q.W)));
-    std::vector<unsigned long long> picks;
-    CDTW_TRY(run_topk(h, d_subject, N, d_avg, d_std, metric == CDTW_EUCLIDEAN, k,
-                      (char*)h->ws, &picks));
-    for (size_t i = 0; i < picks.size(); ++i) {
-        const uint32_t bits = (uint32_t)(picks[i] >> 32);
-        float d;
-        memcpy(&d, &bits, 4);
-        locations[i] = (int64_t)(uint32_t)picks[i];
-        if (distances) distances[i] = metric == CDTW_EUCLIDEAN ? sqrtf(d) : d;
-    }
-    if (found) *found = (int)picks.size();
-    return CDTW_OK;
-}
-
-int cdtw_topk_device(cdtw_handle h, const float* d_subject, int64_t N, const double* d_avg,
-                     const float* d_std, int metric, int k, int64_t* locations,
-                     float* distances, int* found) {
-    if (!h) return CDTW_EINVAL;
-    if (found) *found = 0;
-    if (!h->has_query) return set_error(h, CDTW_EINVAL, "no query set (cdtw_set_query)");
-    const int M = h->q.M;
-    if (!d_subject || !d_avg || !d_std || !locations || k < 1)
-        return set_error(h, CDTW_EINVAL, "bad top-k arguments");
-    if (N < M || N - M + 1 > (int64_t)INT32_MAX)
-        return set_error(h, CDTW_EINVAL, "subject length %lld for M=%d", (long long)N, M);
-    if (M < 11) return set_error(h, CDTW_EUNSUPPORTED, "top-k search needs M >= 11");
-    if (!valid_metric(metric)) return set_error(h, CDTW_EINVAL, "bad metric %d", metric);
-    if (k > (N - M + 1)) k = (int)(N - M + 1);
+    const int64_t Nw = N - M + 1;
+    k = (int)std::min<int64_t>(k, div_up(Nw, M));  // no more windows fit without overlap
     CDTW_CUDA(h, cudaSetDevice(h->device));
     Carver c;
     const size_t o_ws = c.take<char>(topk_device_workspace_bytes(N, M, h->q.W, k));
@@ -466,17 +438,22 @@ int cdtw_topk_device(cdtw_handle h, const float* d_subject, int64_t N, const dou
     int32_t* picks = (int32_t*)(base + o_pk);
     float* pick_d = (float*)(base + o_pd);
     int* cnt = (int*)(base + o_n);
+    int* ctr;
     CDTW_TRY(run_topk_device(h, d_subject, N, d_avg, d_std, metric == CDTW_EUCLIDEAN, k, k,
-                             base + o_ws, nullptr, nullptr, picks, pick_d, cnt, cnt + 1));
-    int hc[2];
+                             base + o_ws, nullptr, nullptr, picks, pick_d, cnt, cnt + 1, &ctr));
+    int hc[2], stage[2];
     std::vector<int32_t> hp(k);
     std::vector<float> hd(k);
     CDTW_CUDA(h, cudaMemcpyAsync(hc, cnt, sizeof(hc), cudaMemcpyDeviceToHost, h->stream));
+    CDTW_CUDA(h, cudaMemcpyAsync(stage, ctr, sizeof(stage), cudaMemcpyDeviceToHost, h->stream));
     CDTW_CUDA(h, cudaMemcpyAsync(hp.data(), picks, sizeof(int32_t) * k, cudaMemcpyDeviceToHost,
                                  h->stream));
     CDTW_CUDA(h, cudaMemcpyAsync(hd.data(), pick_d, sizeof(float) * k, cudaMemcpyDeviceToHost,
                                  h->stream));
     CDTW_CUDA(h, cudaStreamSynchronize(h->stream));
+    h->last_counts[0] = Nw;
+    h->last_counts[1] = stage[0];
+    h->last_counts[2] = stage[1];
     if (hc[1] != 0)
         return set_error(h, CDTW_EUNSUPPORTED,
                          "more windows under the top-k threshold than the hit list holds");
@@ -487,6 +464,12 @@ int cdtw_topk_device(cdtw_handle h, const float* d_subject, int64_t N, const dou
     }
     if (found) *found = n;
     return CDTW_OK;
+}
+
+int cdtw_topk_device(cdtw_handle h, const float* d_subject, int64_t N, const double* d_avg,
+                     const float* d_std, int metric, int k, int64_t* locations,
+                     float* distances, int* found) {
+    return cdtw_topk(h, d_subject, N, d_avg, d_std, metric, k, locations, distances, found);
 }
 
 int cdtw_search_host(cdtw_handle h, const float* h_query, int M, const float* h_subject,

@@ -111,16 +111,12 @@ int search_batched_pipelines(cdtw_handle h, const float* d_subject, int64_t N,
                              const float* h_queries, const std::vector<int>& M,
                              const std::vector<int>& W, int metric, int64_t* locations,
                              float* distances);
-// top-k non-overlapping matches (search.cu)
-size_t topk_workspace_bytes(int64_t N, int M, int W);
-int run_topk(cdtw_handle h, const float* x, int64_t N, const double* mu, const float* sigma,
-             bool euclid, int k, char* ws_base, std::vector<unsigned long long>* picks);
-// the same with every step on the device (graph-capturable); k2 >= k picks
+// top-k non-overlapping matches (search.cu), graph-capturable; k2 >= k picks
 size_t topk_device_workspace_bytes(int64_t N, int M, int W, int k2);
 int run_topk_device(cdtw_handle h, const float* x, int64_t N, const double* mu,
                     const float* sigma, bool euclid, int k, int k2, char* ws_base,
                     const int32_t* prev, const int* prev_n, int32_t* picks, float* pick_d,
-                    int* npicks, int* status);
+                    int* npicks, int* status, int** ctr_out = nullptr);
 // topk_device.cu
 int launch_topk_threshold(cdtw_handle h, const float* sd, int nseg, const float* prev_d,
                           const int* prev_n, int k2, unsigned long long* key, float* t_out);

@@ -26,8 +26,6 @@
 #include "common.cuh"
 
 #include <algorithm>
-#include <set>
-#include <vector>
 
 namespace cdtw {
 
@@ -741,26 +739,9 @@ __global__ void topk_seed_kernel(const float* __restrict__ lbkim, int Nw, int M,
     if (lane == 0) sidx[s] = best == ~0ull ? lo : (int32_t)(uint32_t)best;
 }
 
-__global__ void cands_to_idx_kernel(const Cand* __restrict__ c, int n, int32_t* __restrict__ idx) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) idx[i] = c[i].w;
-}
-
-// Windows whose cDTW is at most T, as packed (distance, window) keys.
-__global__ void collect_kernel(const float* __restrict__ d, const int32_t* __restrict__ idx,
-                               int n, float T, unsigned long long* __restrict__ hits,
-                               int* __restrict__ nh, int cap) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n || !(d[i] <= T)) return;
-    const int at = atomicAdd(nh, 1);
-    if (at < cap) hits[at] = pack_key(d[i], (uint32_t)idx[i]);
-}
-
 struct TopkWs {
     int32_t* sidx;
     float* sd;
-    int32_t* idx;
-    float* d;
     unsigned long long* hits;
     int* nh;
 };
@@ -776,8 +757,6 @@ size_t carve_topk(int64_t N, int64_t Nw, int M, int W, int64_t cap, SearchWs* sw
     const int64_t nseg = div_up(Nw, 2 * (int64_t)M);
     tw->sidx = (int32_t*)take(sizeof(int32_t) * nseg);
     tw->sd = (float*)take(sizeof(float) * nseg);
-    tw->idx = (int32_t*)take(sizeof(int32_t) * Nw);
-    tw->d = (float*)take(sizeof(float) * Nw);
     tw->hits = (unsigned long long*)take(sizeof(unsigned long long) * cap);
     tw->nh = (int*)take(sizeof(int) * 2);
     return off;
@@ -787,116 +766,8 @@ int64_t topk_cap(int64_t Nw) { return std::min<int64_t>(Nw, (int64_t)1 << 24); }
 
 }  // namespace
 
-size_t topk_workspace_bytes(int64_t N, int M, int W) {
-    SearchWs sw;
-    TopkWs tw;
-    const int64_t Nw = N - M + 1;
-    return carve_topk(N, Nw, M, W, topk_cap(Nw), &sw, &tw, nullptr);
-}
-
-// Greedy non-overlapping selection over the (distance, window) keys in
-// ascending order: a window overlapping an accepted one is skipped, and the
-// selection stops at k.  The keys are unique; only the prefix the greedy
-// consumes is ordered: nth_element splits off the next smallest block, which
-// is sorted and scanned, the block doubling until k windows are accepted.
-static void greedy_picks(std::vector<unsigned long long>& hits, int k, int M,
-                         std::vector<unsigned long long>* picks) {
-    std::set<int64_t> taken;
-    picks->clear();
-    size_t lo = 0, block = std::max<size_t>(4096, (size_t)16 * (size_t)k);
-    while (lo < hits.size() && (int)picks->size() < k) {
-        const size_t hi = std::min(hits.size(), lo + block);
-        if (hi < hits.size()) std::nth_element(hits.begin() + lo, hits.begin() + hi, hits.end());
-        std::sort(hits.begin() + lo, hits.begin() + hi);
-        for (size_t i = lo; i < hi && (int)picks->size() < k; ++i) {
-            const unsigned long long key = hits[i];
-            const int64_t w = (int64_t)(uint32_t)key;
-            auto it = taken.lower_bound(w - M + 1);
-            if (it != taken.end() && *it < w + M) continue;  // overlaps an accepted window
-            taken.insert(w);
-            picks->push_back(key);
-        }
-        lo = hi;
-        block *= 2;
-    }
-}
-
-// Top-k non-overlapping matches of the handle's query.  Greedy selection in
-// (distance, window) order with windows overlapping an accepted one skipped.
-// The candidate threshold T is the 2k-th smallest cDTW among the segment
-// seeds: they are pairwise non-overlapping, and each accepted match overlaps
-// at most two of them, so every one of the first k greedy picks has a
-// distance <= T and all windows above T can be pruned.  Host-synchronous.
-int run_topk(cdtw_handle h, const float* x, int64_t N, const double* mu, const float* sigma,
-             bool euclid, int k, char* ws_base, std::vector<unsigned long long>* picks) {
-    const QueryPack& q = h->q;
-    const int M = q.M;
-    const int64_t Nw = N - M + 1;
-    SearchWs ws;
-    TopkWs tw;
-    const int64_t cap = topk_cap(Nw);
-    carve_topk(N, Nw, M, q.W, cap, &ws, &tw, ws_base);
-    const int nseg = (int)div_up(Nw, 2 * (int64_t)M);
-    // 1. LB_Kim of every window, seeds per segment, their exact cDTW
-    CDTW_TRY(launch_lb_kim(h, x, N, mu, sigma, nullptr, Nw, euclid, ws.lbkim, ws.seeds,
-                           ws.bmax));
-    topk_seed_kernel<<<(unsigned)div_up((int64_t)nseg * 32, 256), 256, 0, h->stream>>>(
-        ws.lbkim, (int)Nw, M, nseg, tw.sidx);
-    CDTW_LAUNCH(h, "topk_seed_kernel");
-    CDTW_TRY(launch_cdtw_windows(h, x, N, mu, sigma, tw.sidx, nseg, euclid, tw.sd));
-    std::vector<float> sd(nseg);
-    CDTW_CUDA(h, cudaMemcpyAsync(sd.data(), tw.sd, sizeof(float) * nseg, cudaMemcpyDeviceToHost,
-                                 h->stream));
-    CDTW_CUDA(h, cudaStreamSynchronize(h->stream));
-    float T = INFINITY;
-    if ((int64_t)nseg >= 2 * (int64_t)k) {
-        std::nth_element(sd.begin(), sd.begin() + (2 * k - 1), sd.end());
-        T = sd[2 * k - 1];
-    }
-    // 2. bounds against T (the key holds T as the best-so-far)
-    const unsigned long long tkey = pack_key(T, 0xffffffffu);
-    CDTW_CUDA(h, cudaMemsetAsync(ws.ctr, 0, sizeof(int) * 8, h->stream));
-    CDTW_CUDA(h, cudaMemsetAsync(tw.nh, 0, sizeof(int) * 2, h->stream));
-    CDTW_CUDA(h, cudaMemcpyAsync(ws.key, &tkey, sizeof(tkey), cudaMemcpyHostToDevice, h->stream));
-    const int grid = h->sm_count * 8;
-    compact_kim_kernel<<<grid, 256, 0, h->stream>>>(ws.lbkim, (int)Nw, ws.key, ws.q1, ws.ctr + 0);
-    CDTW_LAUNCH(h, "compact_kim_kernel");
-    CDTW_TRY(launch_keogh(h, x, N, mu, sigma, euclid, ws));
-    int cnt[2];
-    CDTW_CUDA(h, cudaMemcpyAsync(cnt, ws.ctr, sizeof(cnt), cudaMemcpyDeviceToHost, h->stream));
-    CDTW_CUDA(h, cudaStreamSynchronize(h->stream));
-    h->last_counts[0] = Nw;
-    h->last_counts[1] = cnt[0];
-    h->last_counts[2] = cnt[1];
-    // 3. exact cDTW of the survivors, those <= T collected
-    const int ns = cnt[1];
-    if (ns > 0) {
-        cands_to_idx_kernel<<<(unsigned)div_up(ns, 256), 256, 0, h->stream>>>(ws.q2, ns, tw.idx);
-        CDTW_LAUNCH(h, "cands_to_idx_kernel");
-        CDTW_TRY(launch_cdtw_windows(h, x, N, mu, sigma, tw.idx, ns, euclid, tw.d));
-        collect_kernel<<<(unsigned)div_up(ns, 256), 256, 0, h->stream>>>(tw.d, tw.idx, ns, T,
-                                                                        tw.hits, tw.nh, (int)cap);
-        CDTW_LAUNCH(h, "collect_kernel");
-    }
-    int nh = 0;
-    CDTW_CUDA(h, cudaMemcpyAsync(&nh, tw.nh, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
-    CDTW_CUDA(h, cudaStreamSynchronize(h->stream));
-    if (nh > cap)
-        return set_error(h, CDTW_EUNSUPPORTED, "%d windows under the top-k threshold (limit %lld)",
-                         nh, (long long)cap);
-    std::vector<unsigned long long> hits(nh);
-    if (nh > 0) {
-        CDTW_CUDA(h, cudaMemcpyAsync(hits.data(), tw.hits, sizeof(unsigned long long) * nh,
-                                     cudaMemcpyDeviceToHost, h->stream));
-        CDTW_CUDA(h, cudaStreamSynchronize(h->stream));
-    }
-    // 4. greedy non-overlapping selection, lowest (distance, window) first
-    greedy_picks(hits, k, M, picks);
-    return CDTW_OK;
-}
-
-// Workspace of run_topk_device: that of run_topk plus the re-scored previous
-// picks, the threshold and the accepted-window buckets of the greedy.
+// Workspace of run_topk_device: the search's, the seeds and hits, the re-scored
+// previous picks, the threshold and the accepted-window buckets of the greedy.
 namespace {
 struct TopkDevWs {
     float* prev_d;
@@ -928,21 +799,26 @@ size_t topk_device_workspace_bytes(int64_t N, int M, int W, int k2) {
     return carve_topk_device(N, M, W, k2, &sw, &tw, &dw, nullptr);
 }
 
-// The top-k search of run_topk with every step on the device (no host
-// synchronisation, so it can be captured in a CUDA graph): the threshold T
-// is selected on the device (and lowered to the largest re-scored distance
-// of `prev`, a previous set of k2 non-overlapping windows, when *prev_n ==
-// k2), the windows at distance <= T are collected by the early-abandoning
-// search kernels into a hit list, and the greedy selection runs in one block
-// (topk_device.cu).  The greedy continues to k2 picks over the same
-// candidates: the first k (T from 2k of the seeds or of `prev`) are the exact
-// greedy picks; all of them are non-overlapping, which is all the next call's
-// threshold needs.  prev may alias picks and prev_n npicks.  *status: 0, or
-// 1 when more windows than the hit list holds fell under T.
+// Top-k non-overlapping matches of the handle's query: greedy selection in
+// (distance, window) order with windows overlapping an accepted one skipped,
+// every step on the device (no host synchronisation, so it can be captured in
+// a CUDA graph).  The candidate threshold T is the 2k-th smallest cDTW among
+// the segment seeds: they are pairwise non-overlapping, and each accepted match
+// overlaps at most two of them, so every one of the first k greedy picks has a
+// distance <= T and all windows above T can be pruned.  T is selected on the
+// device (and lowered to the largest re-scored distance of `prev`, a previous
+// set of k2 non-overlapping windows, when *prev_n == k2), the windows at
+// distance <= T are collected by the early-abandoning search kernels into a
+// hit list, and the greedy selection runs in one block (topk_device.cu).  It
+// continues to k2 picks over the same candidates: the first k (T from 2k of
+// the seeds or of `prev`) are the exact greedy picks; all of them are
+// non-overlapping, which is all the next call's threshold needs.  prev may
+// alias picks and prev_n npicks.  *status: 0, or 1 when more windows than the
+// hit list holds fell under T.  ctr_out: the stage counts (device).
 int run_topk_device(cdtw_handle h, const float* x, int64_t N, const double* mu,
                     const float* sigma, bool euclid, int k, int k2, char* ws_base,
                     const int32_t* prev, const int* prev_n, int32_t* picks, float* pick_d,
-                    int* npicks, int* status) {
+                    int* npicks, int* status, int** ctr_out) {
     const QueryPack& q = h->q;
     const int M = q.M;
     const int64_t Nw = N - M + 1;
@@ -957,7 +833,7 @@ int run_topk_device(cdtw_handle h, const float* x, int64_t N, const double* mu,
     CDTW_CUDA(h, cudaMemsetAsync(ws.ctr, 0, sizeof(int) * 8, h->stream));
     CDTW_CUDA(h, cudaMemsetAsync(tw.nh, 0, sizeof(int) * 2, h->stream));
     // 1. LB_Kim of every window, one seed per segment, their exact cDTW
-    CDTW_TRY(launch_lb_kim(h, x, N, mu, sigma, nullptr, Nw, euclid, ws.lbkim));
+    CDTW_TRY(launch_lb_kim_all(h, x, N, mu, sigma, euclid, ws.lbkim, ws.seeds, ws.bmax));
     topk_seed_kernel<<<(unsigned)div_up((int64_t)nseg * 32, 256), 256, 0, h->stream>>>(
         ws.lbkim, (int)Nw, M, nseg, tw.sidx);
     CDTW_LAUNCH(h, "topk_seed_kernel");
@@ -981,6 +857,7 @@ int run_topk_device(cdtw_handle h, const float* x, int64_t N, const double* mu,
     // 4. greedy selection
     CDTW_CUDA(h, cudaMemsetAsync(dw.acc, 0xff, sizeof(int) * ((size_t)dw.nbuckets + 2),
                                  h->stream));
+    if (ctr_out) *ctr_out = ws.ctr;
     return launch_topk_greedy(h, tw.hits, tw.nh, (int)cap, k2, M, dw.acc, picks, pick_d, npicks,
                               status);
 }

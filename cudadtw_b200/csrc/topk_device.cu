@@ -23,17 +23,27 @@ constexpr int kSelThreads = 1024;
 constexpr int kGreedyB = 4096;  // keys ordered per round (32 KB of shared memory)
 
 // Index (in an ascending order of n values) of the bucket that holds rank r:
-// on return, *r is the rank inside that bucket.  hist: 256 counts.  Thread 0.
-__device__ int pick_digit(const int* hist, int* r) {
-    int cum = 0;
-    for (int d = 0; d < 256; ++d) {
-        if (cum + hist[d] > *r) {
-            *r -= cum;
-            return d;
-        }
-        cum += hist[d];
+// on return, *r is the rank inside that bucket.  hist: 256 counts.  The lanes
+// of one warp call together, eight buckets each, and all get both (by one
+// thread it was 4 us a digit).
+__device__ __forceinline__ int pick_digit(const int* hist, int* r) {
+    const int lane = threadIdx.x & 31;
+    int sum = 0;
+#pragma unroll
+    for (int d = 0; d < 8; ++d) sum += hist[8 * lane + d];
+    int incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += t;
     }
-    return 255;
+    const unsigned in = __ballot_sync(0xffffffffu, incl > *r);
+    const int src = in ? __ffs(in) - 1 : 31;
+    int left = __shfl_sync(0xffffffffu, *r - (incl - sum), src);
+    int digit = 8 * src;
+    for (; digit < 8 * src + 7 && left >= hist[digit]; ++digit) left -= hist[digit];
+    *r = left;
+    return digit;
 }
 
 // The (r+1)-th smallest of n non-negative floats (their bits order as
@@ -50,10 +60,13 @@ __device__ float select_rank_f32(const float* __restrict__ v, int n, int r, int*
             if ((u & mask) == prefix) atomicAdd(&hist[(u >> shift) & 255u], 1);
         }
         __syncthreads();
-        if (threadIdx.x == 0) *shared_prefix = prefix | ((unsigned)pick_digit(hist, &r) << shift);
+        if (threadIdx.x < 32) {
+            const int digit = pick_digit(hist, &r);
+            if (threadIdx.x == 0) *shared_prefix = prefix | ((unsigned)digit << shift);
+        }
         __syncthreads();
         prefix = *shared_prefix;
-        mask |= 255u << shift;  // (only thread 0's copy of r is used)
+        mask |= 255u << shift;  // (only warp 0's copies of r are used)
         __syncthreads();
     }
     return __uint_as_float(prefix);
@@ -90,12 +103,14 @@ topk_threshold_kernel(const float* __restrict__ sd, int nseg, const float* __res
 }
 
 // Does window w overlap an accepted window?  acc[b + 1]: the accepted
-// window of bucket b (starts bM .. bM + M - 1), or -1.
+// window of bucket b (starts bM .. bM + M - 1), or -1.  The block is the only
+// writer, a barrier between its stores and these loads, so they may come from
+// the SM's L1.
 __device__ __forceinline__ bool overlaps_accepted(const int* acc, int w, int M) {
     const int b = w / M;
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-        const int a = *(const volatile int*)(acc + b + d);  // buckets b-1, b, b+1
+        const int a = acc[b + d];  // buckets b-1, b, b+1
         if (a >= 0 && abs(a - w) < M) return true;
     }
     return false;
@@ -128,8 +143,11 @@ topk_greedy_kernel(const unsigned long long* __restrict__ hits, const int* __res
     __syncthreads();
     unsigned long long lo = 0;  // keys below lo are consumed
     int consumed = 0;
+    // the windows around a match are hits too: about 16 keys a pick first
+    int chunk = min(kGreedyB, max(512, 16 * min(k2, kGreedyB)));
     while (consumed < nh && s_np < k2) {
-        const int take = min(kGreedyB, nh - consumed);
+        const int take = min(chunk, nh - consumed);
+        chunk = kGreedyB;
         // hi = the take-th smallest key >= lo (all of them when they fit)
         unsigned long long hi = ~0ull;
         if (take < nh - consumed) {
@@ -144,7 +162,10 @@ topk_greedy_kernel(const unsigned long long* __restrict__ hits, const int* __res
                         atomicAdd(&hist[(unsigned)(k >> shift) & 255u], 1);
                 }
                 __syncthreads();
-                if (tid == 0) s_pfx = prefix | ((unsigned long long)pick_digit(hist, &r) << shift);
+                if (warp == 0) {
+                    const int digit = pick_digit(hist, &r);
+                    if (lane == 0) s_pfx = prefix | ((unsigned long long)digit << shift);
+                }
                 __syncthreads();
                 prefix = s_pfx;
                 mask |= 255ull << shift;

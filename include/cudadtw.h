@@ -153,11 +153,11 @@ int cdtw_topk(cdtw_handle h, const float* d_subject, int64_t N, const double* d_
               const float* d_std, int metric, int k, int64_t* locations, float* distances,
               int* found);
 
-/* cdtw_topk with every step on the device: the threshold by radix selection,
- * the windows under it collected by the early-abandoning search kernels, the
- * greedy selection in one thread block (the keys ordered only as far as it
- * consumes them).  The same picks as cdtw_topk; one host sync at the end.
- * The steps are those each iteration of cdtw_refine_templates_search runs
+/* The same call by its other name: cdtw_topk runs every step on the device (the
+ * threshold by radix selection, the windows under it collected by the
+ * early-abandoning search kernels, the greedy selection in one thread block,
+ * the keys ordered only as far as it consumes them) with one host sync at the
+ * end.  The steps are those each iteration of cdtw_refine_templates_search runs
  * inside its CUDA graph.  CDTW_EUNSUPPORTED when more than min(N-M+1, 2^24)
  * windows fall under the threshold. */
 int cdtw_topk_device(cdtw_handle h, const float* d_subject, int64_t N, const double* d_avg,
