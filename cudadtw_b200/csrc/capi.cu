@@ -510,16 +510,14 @@ static int ed_run(cdtw_handle h, const double* dq, int M, const double* dx, int6
     Carver c;
     c.off = *used;
     const size_t o_zq = c.take<double>(M);
-    const size_t o_mu = c.take<double>(Nw);
-    const size_t o_sd = c.take<double>(Nw);
+    const size_t o_rs = c.take<double>(Nw);
     *used = c.off;
     if (!base) return CDTW_OK;
     double* zq = (double*)(base + o_zq);
-    double* mu = (double*)(base + o_mu);
-    double* sd = (double*)(base + o_sd);
+    double* rs = (double*)(base + o_rs);
     CDTW_TRY(launch_znorm64(h, dq, M, zq));
-    CDTW_TRY(launch_avg_std64(h, dx, N, M, mu, sd));
-    return launch_ed(h, dx, N, zq, M, sd, dout);
+    CDTW_TRY(launch_rstd64(h, dx, N, M, rs));
+    return launch_ed(h, dx, N, zq, M, rs, dout);
 }
 
 int ed_all_windows(cdtw_handle h, const double* d_query, int M, const double* d_subject,

@@ -378,7 +378,7 @@ __device__ __forceinline__ void report_window(unsigned long long* key, const Hit
 
 int launch_avg_std(cdtw_handle h, const float* x, int64_t N, int M, double* mu, float* sigma);
 int launch_avg_std64(cdtw_handle h, const float* x, int64_t N, int M, double* mu, double* sigma);
-int launch_avg_std64(cdtw_handle h, const double* x, int64_t N, int M, double* mu, double* sigma);
+int launch_rstd64(cdtw_handle h, const double* x, int64_t N, int M, double* rs);  // 1 / sigma
 // Exact FP64 argmin (lowest index on ties) of d[0..n): block partials then one
 // final block; the result (value, index) lands in *res.
 struct ArgMin64 {
@@ -390,7 +390,7 @@ int launch_argmin64(cdtw_handle h, const double* d, int64_t n, ArgMin64* partial
 size_t argmin64_partials(int64_t n);
 int launch_znorm64(cdtw_handle h, const double* q, int M, double* zq);
 int launch_ed(cdtw_handle h, const double* x, int64_t N, const double* zq, int M,
-              const double* sigma, double* out);
+              const double* rs, double* out);  // rs: 1 / sigma per window
 int launch_ldtw(cdtw_handle h, const float* x, int64_t N, const double* mu, const double* sigma,
                 bool euclid, double* out);
 // The reference's FP32 LDTW (ztsh2_ldtw / tsh2_ldtw arithmetic); qwork: M

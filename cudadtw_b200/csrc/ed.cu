@@ -10,7 +10,8 @@
 // slides them over the query with the window samples in registers (one new
 // sample load per query step for 8 FMAs), the query and the series tile staged
 // in shared memory (padded one double per eight so the eight-apart thread
-// reads do not collide in banks), then an exact FP64 argmin.  No FFT, no sort.
+// reads do not collide in banks), with 1 / sigma from the statistics kernel,
+// then an exact FP64 argmin.  No FFT, no sort.
 #include "common.cuh"
 
 #include <algorithm>
@@ -25,46 +26,90 @@ constexpr int kEdTile = kEdThreads * kEdR;         // windows per block
 constexpr int kEdK = 256;                          // query positions per chunk
 constexpr int kEdSpan = kEdTile + kEdK + kEdR;     // samples staged per chunk
 constexpr int kEdXs = kEdSpan + (kEdSpan >> 3) + 1;  // with one pad per eight
+constexpr int kEdStage = kEdXs + kEdK;               // doubles of a stage: samples, query chunk
 
 __device__ __forceinline__ int pad8(int i) { return i + (i >> 3); }
 
+// dst = *src, or 0 without reading where !in (8 bytes, asynchronously).
+__device__ __forceinline__ void copy8(double* dst, const double* src, bool in) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src),
+                 "r"(in ? 8 : 0)
+                 : "memory");
+}
+
+// rs: 1 / sigma per window.  Bound by the FP64 pipe (2^21 windows, M = 256:
+// 5.4e8 multiply-adds, 29 us at 64 a cycle and SM).  Persistent blocks go
+// through (tile, query chunk) stages with the next stage's copies in flight
+// under the current one's arithmetic: with a block per tile every wave of
+// blocks loaded together, computed together and divided by sigma together (60
+// us; with the statistics pass 81, now 67).
 __global__ void __launch_bounds__(kEdThreads)
 ed_kernel(const double* __restrict__ x, int64_t N, const double* __restrict__ zq, int M,
-          int64_t Nw, const double* __restrict__ sigma, double* __restrict__ out) {
-    __shared__ double xs[kEdXs];
-    __shared__ double qs[kEdK];
-    const int64_t t0 = (int64_t)blockIdx.x * kEdTile;
+          int64_t Nw, const double* __restrict__ rs, double* __restrict__ out) {
+    extern __shared__ double esm[];  // two stages
     const int t = threadIdx.x;
-    double acc[kEdR];
-#pragma unroll
-    for (int r = 0; r < kEdR; ++r) acc[r] = 0.0;
-    for (int k0 = 0; k0 < M; k0 += kEdK) {
-        const int kn = min(kEdK, M - k0);
-        __syncthreads();
+    const int64_t tiles = (Nw + kEdTile - 1) / kEdTile;
+    const int chunks = (M + kEdK - 1) / kEdK;
+    auto stage_in = [&](int64_t tile, int chunk, double* xs) {
+        const int64_t g0 = tile * kEdTile + (int64_t)chunk * kEdK;
         for (int i = t; i < kEdSpan; i += kEdThreads) {
-            const int64_t g = t0 + k0 + i;
-            xs[pad8(i)] = g < N ? x[g] : 0.0;
+            const bool in = g0 + i < N;
+            copy8(xs + pad8(i), x + (in ? g0 + i : 0), in);
         }
-        for (int i = t; i < kEdK; i += kEdThreads) qs[i] = i < kn ? zq[k0 + i] : 0.0;
-        __syncthreads();
-        const int b = t * kEdR;
-        double xr[kEdR];
+        double* qs = xs + kEdXs;
+        for (int i = t; i < kEdK; i += kEdThreads) {
+            const int k = chunk * kEdK + i;
+            copy8(qs + i, zq + (k < M ? k : 0), k < M);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    int64_t tile = blockIdx.x;
+    if (tile >= tiles) return;
+    stage_in(tile, 0, esm);
+    int buf = 0;
+    for (; tile < tiles; tile += gridDim.x) {
+        double acc[kEdR], rsv[kEdR];
+        const int64_t w0 = tile * kEdTile + (int64_t)t * kEdR;
 #pragma unroll
-        for (int r = 0; r < kEdR; ++r) xr[r] = xs[pad8(b + r)];
-        for (int k = 0; k < kn; k += kEdR) {
-#pragma unroll
-            for (int u = 0; u < kEdR; ++u) {
-                const double q = qs[k + u];  // zero beyond kn
-#pragma unroll
-                for (int r = 0; r < kEdR; ++r) acc[r] = fma(q, xr[(r + u) % kEdR], acc[r]);
-                xr[u] = xs[pad8(b + k + u + kEdR)];  // sample b+k+u+R replaces b+k+u
+        for (int r = 0; r < kEdR; ++r) acc[r] = 0.0;
+        for (int chunk = 0; chunk < chunks; ++chunk) {
+            const bool last = chunk + 1 == chunks;
+            const int64_t next = last ? tile + gridDim.x : tile;
+            __syncthreads();  // the other buffer is read
+            if (next < tiles) {
+                stage_in(next, last ? 0 : chunk + 1, esm + (buf ^ 1) * kEdStage);
+                asm volatile("cp.async.wait_group 1;" ::: "memory");
+            } else {
+                asm volatile("cp.async.wait_group 0;" ::: "memory");
             }
-        }
-    }
+            if (last) {
 #pragma unroll
-    for (int r = 0; r < kEdR; ++r) {
-        const int64_t w = t0 + t * kEdR + r;
-        if (w < Nw) out[w] = 2.0 * M - 2.0 * acc[r] / sigma[w];
+                for (int r = 0; r < kEdR; ++r) rsv[r] = rs[min(w0 + r, Nw - 1)];
+            }
+            __syncthreads();
+            const double* xs = esm + buf * kEdStage;
+            const double* qs = xs + kEdXs;
+            const int kn = min(kEdK, M - chunk * kEdK);
+            const double* xb = xs + (kEdR + 1) * t;  // pad8(8 t)
+            double xr[kEdR];
+#pragma unroll
+            for (int r = 0; r < kEdR; ++r) xr[r] = xb[r];
+            for (int k = 0; k < kn; k += kEdR) {
+                xb += kEdR + 1;
+#pragma unroll
+                for (int u = 0; u < kEdR; ++u) {
+                    const double q = qs[k + u];  // zero beyond kn
+#pragma unroll
+                    for (int r = 0; r < kEdR; ++r) acc[r] = fma(q, xr[(r + u) % kEdR], acc[r]);
+                    xr[u] = xb[u];  // sample 8t + k + 8 + u replaces 8t + k + u
+                }
+            }
+            buf ^= 1;
+        }
+#pragma unroll
+        for (int r = 0; r < kEdR; ++r)
+            if (w0 + r < Nw) out[w0 + r] = fma(-2.0 * acc[r], rsv[r], 2.0 * M);
     }
 }
 
@@ -178,10 +223,17 @@ int launch_znorm64(cdtw_handle h, const double* q, int M, double* zq) {
 }
 
 int launch_ed(cdtw_handle h, const double* x, int64_t N, const double* zq, int M,
-              const double* sigma, double* out) {
+              const double* rs, double* out) {
     const int64_t Nw = N - M + 1;
-    ed_kernel<<<(unsigned)div_up(Nw, kEdTile), kEdThreads, 0, h->stream>>>(x, N, zq, M, Nw, sigma,
-                                                                          out);
+    const size_t smem = 2 * kEdStage * sizeof(double);
+    CDTW_CUDA(h, cudaFuncSetAttribute((const void*)ed_kernel,
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    int per_sm = 0;
+    CDTW_CUDA(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)ed_kernel,
+                                                               kEdThreads, smem));
+    const unsigned blocks = (unsigned)std::min<int64_t>(
+        div_up(Nw, kEdTile), (int64_t)std::max(per_sm, 1) * h->sm_count);
+    ed_kernel<<<blocks, kEdThreads, smem, h->stream>>>(x, N, zq, M, Nw, rs, out);
     CDTW_LAUNCH(h, "ed_kernel");
     return CDTW_OK;
 }

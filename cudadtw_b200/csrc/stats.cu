@@ -29,10 +29,10 @@ __device__ __forceinline__ double warp_sum(double v) {
 
 // Windows of any length, a warp per run of kStatsWarpWindows: serves the
 // lengths above kTileMaxM, whose tile would not fit shared memory.
-template <class XT, class ST>
+template <class XT, class ST, bool INV>
 __global__ void __launch_bounds__(kStatsBlock)
 avg_std_long_kernel(const XT* __restrict__ x, int64_t N, int M, double* __restrict__ mu,
-               ST* __restrict__ sigma) {
+                    ST* __restrict__ sigma) {
     // The warp's run of kStatsWarpWindows windows is split into kStatsSub
     // sub-runs, each with its own shift c and starting sums; their scans are
     // interleaved round by round (independent shuffle / FP64 chains).
@@ -109,8 +109,9 @@ avg_std_long_kernel(const XT* __restrict__ x, int64_t N, int M, double* __restri
             if (wv[u] < Nw) {
                 const double m1 = w1 * invM;
                 const double var = w2 * invM - m1 * m1;
-                mu[wv[u]] = c[u] + m1;
-                sigma[wv[u]] = var > 0.0 ? (ST)sqrt(var) : (ST)1;
+                if (mu) mu[wv[u]] = c[u] + m1;
+                const double sd = var > 0.0 ? sqrt(var) : 1.0;
+                sigma[wv[u]] = INV ? (ST)(1.0 / sd) : (ST)sd;
             }
             s1[u] += __shfl_sync(0xffffffffu, i1[u], 31);
             s2[u] += __shfl_sync(0xffffffffu, i2[u], 31);
@@ -122,10 +123,13 @@ avg_std_long_kernel(const XT* __restrict__ x, int64_t N, int M, double* __restri
 // (s0 = v * rsqrt(v)) and one Heron step whose residual v - s0^2 is taken in
 // FP64, so the result is the FP64 root rounded to FP32 but for ties within
 // 1e-7 ulp, at a fraction of the FP64 square root's instructions.
+template <bool INV>
 __device__ __forceinline__ double std_of(double var, double) {
-    return var > 0.0 ? sqrt(var) : 1.0;
+    return var > 0.0 ? (INV ? rsqrt(var) : sqrt(var)) : 1.0;
 }
+template <bool INV>
 __device__ __forceinline__ float std_of(double var, float) {
+    static_assert(!INV, "the reciprocal is FP64 only");
     const float v = (float)var;
     if (!(v > 1e-30f && v < 1e30f)) return var > 0.0 ? (float)sqrt(var) : 1.0f;
     float y;
@@ -277,7 +281,8 @@ __device__ __forceinline__ void tile_out(T* z, const T (&v)[kTileR], T* __restri
     }
 }
 
-template <class XT, class ST>
+// mu may be null (not wanted); INV: sigma takes 1 / sigma.
+template <class XT, class ST, bool INV>
 __global__ void __launch_bounds__(kTileThreads, 6)
 avg_std_kernel(const XT* __restrict__ x, int64_t N, int M, double* __restrict__ mu,
                ST* __restrict__ sigma) {
@@ -383,7 +388,7 @@ avg_std_kernel(const XT* __restrict__ x, int64_t N, int M, double* __restrict__ 
         const double m1 = w1 * invM;
         const double var = fma(-m1, m1, w2 * invM);
         om[r] = c + m1;
-        os[r] = std_of(var, ST());
+        os[r] = std_of<INV>(var, ST());
         again |= var >= lost ? 0u : 1u << r;
         const double vin = (double)in[r] - c, d = vin - v[r];
         w1 += d;
@@ -395,14 +400,15 @@ avg_std_kernel(const XT* __restrict__ x, int64_t N, int M, double* __restrict__ 
             if ((again >> r & 1u) && t0 + kTileR * t + r < Nw) {
                 const double2 q = tile_window(xs, kTileR * t + r, M);
                 om[r] = q.x;
-                os[r] = std_of(q.y, ST());
+                os[r] = std_of<INV>(q.y, ST());
             }
         }
     }
     // the samples and prefixes make room for the sigmas, these for the means
     tile_out(reinterpret_cast<ST*>(tsm), os, sigma + t0, (int)min((int64_t)kTileWindows, Nw - t0));
-    tile_out(reinterpret_cast<double*>(tsm), om, mu + t0,
-             (int)min((int64_t)kTileWindows, Nw - t0));
+    if (mu)
+        tile_out(reinterpret_cast<double*>(tsm), om, mu + t0,
+                 (int)min((int64_t)kTileWindows, Nw - t0));
 }
 
 // One block prepares the query pack: FP64 two-pass z-normalisation (the
@@ -510,37 +516,38 @@ prepare_queries_kernel(const float* __restrict__ raw, const int64_t* __restrict_
 
 }  // namespace
 
-template <class XT, class ST>
+template <bool INV, class XT, class ST>
 static int launch_stats(cdtw_handle h, const XT* x, int64_t N, int M, double* mu, ST* sigma) {
     const int64_t Nw = N - M + 1;
     if (M > kTileMaxM) {
         const int64_t blocks = div_up(div_up(Nw, kStatsWarpWindows), kStatsBlock / 32);
-        avg_std_long_kernel<XT, ST><<<(unsigned)blocks, kStatsBlock, 0, h->stream>>>(x, N, M, mu,
+        avg_std_long_kernel<XT, ST, INV><<<(unsigned)blocks, kStatsBlock, 0, h->stream>>>(x, N, M, mu,
                                                                                     sigma);
         CDTW_LAUNCH(h, "avg_std_long_kernel");
         return CDTW_OK;
     }
     const size_t smem = tile_smem<XT, ST>(M);
     if (smem > 48 * 1024)
-        CDTW_CUDA(h, cudaFuncSetAttribute((const void*)avg_std_kernel<XT, ST>,
+        CDTW_CUDA(h, cudaFuncSetAttribute((const void*)avg_std_kernel<XT, ST, INV>,
                                           cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int)smem));
-    avg_std_kernel<XT, ST><<<(unsigned)div_up(Nw, kTileWindows), kTileThreads, smem, h->stream>>>(
-        x, N, M, mu, sigma);
+    avg_std_kernel<XT, ST, INV>
+        <<<(unsigned)div_up(Nw, kTileWindows), kTileThreads, smem, h->stream>>>(x, N, M, mu, sigma);
     CDTW_LAUNCH(h, "avg_std_kernel");
     return CDTW_OK;
 }
 
 int launch_avg_std(cdtw_handle h, const float* x, int64_t N, int M, double* mu, float* sigma) {
-    return launch_stats(h, x, N, M, mu, sigma);
+    return launch_stats<false>(h, x, N, M, mu, sigma);
 }
 
-// FP64 sigma (ED and LDTW paths), float32 or float64 series.
+// FP64 sigma (LDTW).
 int launch_avg_std64(cdtw_handle h, const float* x, int64_t N, int M, double* mu, double* sigma) {
-    return launch_stats(h, x, N, M, mu, sigma);
+    return launch_stats<false>(h, x, N, M, mu, sigma);
 }
-int launch_avg_std64(cdtw_handle h, const double* x, int64_t N, int M, double* mu, double* sigma) {
-    return launch_stats(h, x, N, M, mu, sigma);
+// 1 / sigma alone (ED).
+int launch_rstd64(cdtw_handle h, const double* x, int64_t N, int M, double* rs) {
+    return launch_stats<true>(h, x, N, M, (double*)nullptr, rs);
 }
 
 int launch_prepare_queries(cdtw_handle h, const float* raw, const int64_t* offs,
