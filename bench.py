@@ -286,8 +286,8 @@ def run_ours(args, rank: int, world: int, local_rank: int) -> None:
                         "h2d_bytes_per_step": len(bands) * (x.nbytes + q.nbytes),
                         "d2h_bytes_per_step": len(bands) * nw * 4},
                 "roofline": {"bound": "alu",
-                             "kernel": "cdtw_regc_kernel<12,EU,4> (W=12) + "
-                                       "cdtw_regc_kernel<25,EU,3> (W=25)",
+                             "kernel": "cdtw_regc_kernel<12,EU,2> (W=12) + "
+                                       "cdtw_regc_kernel<25,EU,2> (W=25)",
                              "achieved": ach, "peak": peak / 1e9, "unit": "GCUPS",
                              "frac": ach / (peak / 1e9),
                              # DRAM bytes (read + write) of one launch of this workload

@@ -18,7 +18,7 @@ batch_reg_kernel(const BatchArgs b) {
     extern __shared__ __align__(16) unsigned char smem[];
     const TileSmem ts = carve_tile(smem, b.tmax, b.mmax);
     float4* sq4 = ts.tail;                             // lq4max (of 4 * lq4max)
-    float2* senv = (float2*)(sq4 + 4 * b.lq4max);      // mmax
+    float2* senv = (float2*)(sq4 + 4 * b.lq4max);      // reg_env_len(mmax)
     __shared__ int s_item, s_na, s_nb, s_next;
     const int tid = threadIdx.x, lane = tid & 31;
     int q, tile;
@@ -27,7 +27,7 @@ batch_reg_kernel(const BatchArgs b) {
         const BatchQ& Q = b.qs[q];
         const int M = Q.sa.M;
         for (int e = tid; e < Q.lq4; e += kBatchThreads) sq4[e] = Q.qpad4[e];
-        for (int e = tid; e < M; e += kBatchThreads) senv[e] = Q.env[e];
+        reg_stage_env(senv, Q.env, M);
         const int t0 = tile * Q.T;
         const int Tq = min(Q.T, Q.Nw - t0);
         tile_front<EU>(b.x, Q, t0, Tq, ts, &s_na, &s_nb);

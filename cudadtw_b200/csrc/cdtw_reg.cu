@@ -96,7 +96,7 @@ int launch_cdtw_search(cdtw_handle h, const float* x, int64_t N, const double* m
                                         sink);
     RegSearchKernel k = euclid ? reg_kernels().seu[q.W] : reg_kernels().smh[q.W];
     const int lq4 = q.lq / 4;
-    const size_t smem = (size_t)q.lq * sizeof(float) + (size_t)q.M * sizeof(float2);
+    const size_t smem = (size_t)q.lq * sizeof(float) + (size_t)reg_env_len(q.M) * sizeof(float2);
     CDTW_CUDA(h, cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)smem));
     int per_sm = 0;

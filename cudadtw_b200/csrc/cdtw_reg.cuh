@@ -115,6 +115,28 @@ __device__ __forceinline__ void reg_rows4(float (&p)[NW][2 * W + 2], const float
     }
 }
 
+// Samples j .. j+3 of xw, those past `last` clamped to it (one branch instead
+// of four clamps; it is the same for the whole warp but at a stream's end).
+__device__ __forceinline__ void reg_load4(float* v, const float* __restrict__ xw, int j,
+                                          int last) {
+    if (j + 3 <= last) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) v[u] = __ldg(xw + j + u);
+    } else {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) v[u] = __ldg(xw + min(j + u, last));
+    }
+}
+
+// The query envelope in shared memory, as the search reads it: four rows a
+// group, (-inf, +inf) past the query (no bound there).  Holds reg_env_len(M).
+__host__ __device__ inline int reg_env_len(int M) { return (M + 3) / 4 * 4; }
+__device__ __forceinline__ void reg_stage_env(float2* senv, const float2* __restrict__ qenv,
+                                              int M) {
+    for (int e = threadIdx.x; e < reg_env_len(M); e += blockDim.x)
+        senv[e] = e < M ? qenv[e] : make_float2(-CDTW_INF, CDTW_INF);
+}
+
 template <int W, int NW>
 __device__ __forceinline__ void reg_init(float (&p)[NW][2 * W + 2]) {
 #pragma unroll
@@ -160,8 +182,7 @@ cdtw_reg_kernel(const float* __restrict__ x, const double* __restrict__ mu,
         nm[v] = make_norm(mu[w], sigma[w]);
         xw[v] = x + w;
         res[v] = CDTW_INF;
-#pragma unroll
-        for (int r = 0; r < 4; ++r) xn[v][r] = __ldg(xw[v] + min(r, M - 1));
+        reg_load4(xn[v], xw[v], 0, M - 1);
     }
     float p[NW][2 * W + 2];
     reg_init<W, NW>(p);
@@ -170,10 +191,8 @@ cdtw_reg_kernel(const float* __restrict__ x, const double* __restrict__ mu,
 #pragma unroll
         for (int v = 0; v < NW; ++v) {
 #pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                z[v][r] = znorm(nm[v], xn[v][r]);
-                xn[v][r] = __ldg(xw[v] + min(j0 + 4 + r, M - 1));
-            }
+            for (int r = 0; r < 4; ++r) z[v][r] = znorm(nm[v], xn[v][r]);
+            reg_load4(xn[v], xw[v], j0 + 4, M - 1);
         }
         reg_rows4<W, EU, NW, true>(p, z, sq4 + (j0 >> 2), M - 1 - j0, res);
     }
@@ -229,8 +248,7 @@ cdtw_regc_kernel(const float* __restrict__ x, const double* __restrict__ mu,
     int j0 = 0;
     for (; j0 + 4 < M; j0 += 4) {
         float nx[4], z[NW][4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) nx[i] = __ldg(xb + min(j0 + NX + i, xlast));
+        reg_load4(nx, xb, j0 + NX, xlast);
         samples(z);
         reg_rows4<W, EU, NW, false>(p, z, sq4 + (j0 >> 2), 0, res);
 #pragma unroll
@@ -281,30 +299,30 @@ __device__ __forceinline__ float reg_window_dtw(const float4* sq4, const float2*
     // wider bands leave no registers for it)
     constexpr bool kAhead = W <= 64;
     float xn[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) xn[u] = kAhead ? __ldg(xw + min(u, M - 1)) : 0.f;
+    if (kAhead) reg_load4(xn, xw, 0, M - 1);
     for (int j0 = 0; j0 < M; j0 += 4) {
         float xc[4];
+        if constexpr (kAhead) {
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            if constexpr (kAhead) {
-                xc[u] = xn[u];
-                xn[u] = __ldg(xw + min(j0 + 4 + u, M - 1));
-            } else {
-                xc[u] = __ldg(xw + min(j0 + u, M - 1));
-            }
+            for (int u = 0; u < 4; ++u) xc[u] = xn[u];
+            reg_load4(xn, xw, j0 + 4, M - 1);
+        } else {
+            reg_load4(xc, xw, j0, M - 1);
         }
         const bool check = (j0 & 7) == 4 && j0 + 3 < M - 1;  // rows j0..j0+3 are all real rows
         // W <= 64: the best-so-far is read before the group's cells
         const float bsf_early = (kAhead && check) ? load_bsf(key) : 0.f;
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int j = j0 + u;
+        for (int u = 0; u < 4; u += 2) {
+            // forward LB_Keogh terms of these data rows (query envelope there;
+            // (-inf, +inf) past row M - 1)
+            const float4 e = reinterpret_cast<const float4*>(senv)[(j0 + u) >> 1];
             z[0][u] = znorm(nm, xc[u]);
-            // forward LB_Keogh term of this data row (query envelope at j)
-            const float2 e = senv[min(j, M - 1)];
-            const float dl = max3f(z[0][u] - e.y, e.x - z[0][u], 0.f);
-            pre += (j < M) ? (EU ? dl * dl : dl) : 0.f;
+            z[0][u + 1] = znorm(nm, xc[u + 1]);
+            const float d0 = max3f(z[0][u] - e.y, e.x - z[0][u], 0.f);
+            const float d1 = max3f(z[0][u + 1] - e.w, e.z - z[0][u + 1], 0.f);
+            pre += EU ? d0 * d0 : d0;
+            pre += EU ? d1 * d1 : d1;
         }
         reg_rows4<W, EU, 1, true>(p, z, sq4 + (j0 >> 2), M - 1 - j0, res);
         if (check) {
@@ -334,7 +352,7 @@ cdtw_reg_search_kernel(const float* __restrict__ x, const double* __restrict__ m
     extern __shared__ float4 sq4[];
     float2* senv = (float2*)(sq4 + lq4);
     for (int e = threadIdx.x; e < lq4; e += blockDim.x) sq4[e] = qpad4[e];
-    for (int e = threadIdx.x; e < M; e += blockDim.x) senv[e] = qenv[e];
+    reg_stage_env(senv, qenv, M);
     __syncthreads();
     const int lane = threadIdx.x & 31;
     const int n = *(const volatile int*)count;
