@@ -144,13 +144,15 @@ topk_greedy_kernel(const unsigned long long* __restrict__ hits, const int* __res
     unsigned long long lo = 0;  // keys below lo are consumed
     int consumed = 0;
     // the windows around a match are hits too: about 16 keys a pick first
-    int chunk = min(kGreedyB, max(512, 16 * min(k2, kGreedyB)));
+    int chunk = min(3 * kGreedyB / 4, max(512, 16 * min(k2, kGreedyB)));
     while (consumed < nh && s_np < k2) {
         const int take = min(chunk, nh - consumed);
-        chunk = kGreedyB;
-        // hi = the take-th smallest key >= lo (all of them when they fit)
+        chunk = 3 * kGreedyB / 4;
+        // hi: a bound with at least `take` and at most kGreedyB keys in [lo, hi]
+        // (all of them when they fit).  A digit's bucket that fits whole ends
+        // the selection: two or three passes over the hits, not eight.
         unsigned long long hi = ~0ull;
-        if (take < nh - consumed) {
+        if (nh - consumed > kGreedyB) {
             unsigned long long prefix = 0, mask = 0;
             int r = take - 1;
             for (int shift = 56; shift >= 0; shift -= 8) {
@@ -164,16 +166,21 @@ topk_greedy_kernel(const unsigned long long* __restrict__ hits, const int* __res
                 __syncthreads();
                 if (warp == 0) {
                     const int digit = pick_digit(hist, &r);
-                    if (lane == 0) s_pfx = prefix | ((unsigned long long)digit << shift);
+                    if (lane == 0) {
+                        s_pfx = prefix | ((unsigned long long)digit << shift);
+                        s_cnt = take - 1 - r + hist[digit];  // keys up to the bucket's end
+                    }
                 }
                 __syncthreads();
                 prefix = s_pfx;
                 mask |= 255ull << shift;
+                const bool whole = s_cnt <= kGreedyB;
                 __syncthreads();
+                if (whole) break;
             }
-            hi = prefix;
+            hi = prefix | ~mask;
         }
-        // gather the keys in [lo, hi] (exactly `take`, keys are unique), sort
+        // gather the keys in [lo, hi], sort
         if (tid == 0) s_cnt = 0;
         __syncthreads();
         for (int i = tid; i < nh; i += kSelThreads) {
@@ -257,7 +264,7 @@ topk_greedy_kernel(const unsigned long long* __restrict__ hits, const int* __res
             }
             __syncthreads();
         }
-        consumed += take;
+        consumed += cnt;
         lo = hi + 1;
         __syncthreads();
     }
