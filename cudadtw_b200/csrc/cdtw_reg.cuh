@@ -46,19 +46,6 @@ namespace {
 constexpr int kRegBlock = 128;
 constexpr int kMaxRegW = 106;  // the widest band that 255 registers hold without spills
 
-// (x, y) as a packed FP32 pair, and the two differences of two pairs.
-__device__ __forceinline__ unsigned long long pack2(float x, float y) {
-    unsigned long long r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
-    return r;
-}
-__device__ __forceinline__ void sub2(unsigned long long a, unsigned long long b, float& lo,
-                                     float& hi) {
-    unsigned long long r;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(r));
-}
-
 // Rows j .. j+3 of NW windows: p holds row j-1 (p[v][B] = +inf) and becomes
 // row j+3; z[v][r] is window v's sample of row j + r, qr the padded query from
 // element j (16-byte aligned; reads up to 2W + 7 further).  Step s takes row r

@@ -216,19 +216,45 @@ __device__ __forceinline__ float znorm(const Norm& n, float x) {
 // the search from the front part alone, the back part computed only where
 // the front part passes, was measured: its seeds are poor enough that the
 // first best-so-far prunes almost nothing on some queries.)
+//
+// The differences of a row come packed, (s[0], s[1]) and (s[2], s[3]) less the
+// query value twice and s[4] alone: the cells are bound by register operands
+// (cdtw_reg.cuh), and the query pairs stay in registers over a lane's windows.
+__device__ __forceinline__ unsigned long long pack2(float x, float y) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+    return r;
+}
+// The two differences of packed pairs, a - b.
+__device__ __forceinline__ void sub2(unsigned long long a, unsigned long long b, float& lo,
+                                     float& hi) {
+    unsigned long long r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(r));
+}
+// d[k] = q - s[k] (its sign does not matter to either cost).
+__device__ __forceinline__ void lb_kim_row(const float* s, float q, float (&d)[5]) {
+    const unsigned long long q2 = pack2(q, q);
+    sub2(pack2(s[0], s[1]), q2, d[0], d[1]);
+    sub2(pack2(s[2], s[3]), q2, d[2], d[3]);
+    d[4] = s[4] - q;
+}
+
 template <bool EU>
 __device__ __forceinline__ float lb_kim_front(const float* s, const float* q) {
     auto lp = [](float d) { return EU ? d * d : fabsf(d); };
-    float F[5], G[5];
-    F[0] = lp(q[0] - s[0]);
+    float F[5], G[5], d[5];
+    lb_kim_row(s, q[0], d);
+    F[0] = lp(d[0]);
 #pragma unroll
-    for (int k = 1; k < 5; ++k) F[k] = lp(q[0] - s[k]) + F[k - 1];
+    for (int k = 1; k < 5; ++k) F[k] = lp(d[k]) + F[k - 1];
     float mem = F[4];
 #pragma unroll
     for (int r = 1; r < 5; ++r) {
-        G[0] = lp(q[r] - s[0]) + F[0];
+        lb_kim_row(s, q[r], d);
+        G[0] = lp(d[0]) + F[0];
 #pragma unroll
-        for (int k = 1; k < 5; ++k) G[k] = lp(q[r] - s[k]) + min3f(G[k - 1], F[k - 1], F[k]);
+        for (int k = 1; k < 5; ++k) G[k] = lp(d[k]) + min3f(G[k - 1], F[k - 1], F[k]);
         mem = fminf(mem, G[4]);
 #pragma unroll
         for (int k = 0; k < 5; ++k) F[k] = G[k];
@@ -242,14 +268,16 @@ __device__ __forceinline__ float lb_kim_front(const float* s, const float* q) {
 template <bool EU>
 __device__ __forceinline__ float lb_kim_back(const float* s, const float* q) {
     auto lp = [](float d) { return EU ? d * d : fabsf(d); };
-    float F[5], G[5];
+    float F[5], G[5], d[5];
+    lb_kim_row(s, q[0], d);
 #pragma unroll
-    for (int k = 0; k < 5; ++k) F[k] = lp(q[0] - s[k]);
+    for (int k = 0; k < 5; ++k) F[k] = lp(d[k]);
 #pragma unroll
     for (int r = 1; r < 5; ++r) {
-        G[0] = lp(q[r] - s[0]);
+        lb_kim_row(s, q[r], d);
+        G[0] = lp(d[0]);
 #pragma unroll
-        for (int k = 1; k < 5; ++k) G[k] = lp(q[r] - s[k]) + min3f(G[k - 1], F[k - 1], F[k]);
+        for (int k = 1; k < 5; ++k) G[k] = lp(d[k]) + min3f(G[k - 1], F[k - 1], F[k]);
 #pragma unroll
         for (int k = 0; k < 5; ++k) F[k] = G[k];
     }
