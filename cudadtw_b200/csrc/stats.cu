@@ -159,10 +159,10 @@ __device__ __forceinline__ float std_of(double var, float) {
 // Bound: HBM (16 bytes a window, 82 us at 2^25 windows and 6546 GB/s) if the
 // latencies of a block's phases were hidden; 72 instructions a window, 24
 // warps per SM.  Six blocks per SM (80 registers, 100 bytes spilled) measured
-// best: 4 / 5 / 6 / 7 / 8 blocks 198 / 169 / 156 / 161 / 168 us at 2^25
-// windows, M = 512, and 10 us at 2^20 windows, M = 128.  Before (a warp per
-// 2048 windows, scans of 32 windows a round): 196 and 22 us, the latter the
-// latency of its serial rounds.
+// best (5 / 6 / 7: 146 / 144 / 144 us at 2^25 windows, M = 512), the samples
+// copied asynchronously (156 us through registers).  2^20 windows, M = 128: 10
+// us.  Before (a warp per 2048 windows, scans of 32 windows a round): 196 and
+// 22 us, the latter the latency of its serial rounds.
 constexpr int kTileThreads = 128;
 constexpr int kTileR = 16;                                // windows per thread, samples per chunk
 constexpr int kTileWindows = kTileThreads * kTileR;       // 2048
@@ -306,8 +306,11 @@ avg_std_kernel(const XT* __restrict__ x, int64_t N, int M, double* __restrict__ 
     if ((reinterpret_cast<uintptr_t>(x) & 15) == 0) {  // t0 is a multiple of 2048
         i0 = have / V * V;
         for (int i = V * t; i < i0; i += V * kTileThreads)
-            *reinterpret_cast<int4*>(xs + tile_at<XT>(i)) =
-                *reinterpret_cast<const int4*>(xt + i);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                             (unsigned)__cvta_generic_to_shared(xs + tile_at<XT>(i))),
+                         "l"(xt + i)
+                         : "memory");
+        asm volatile("cp.async.wait_all;" ::: "memory");
     }
     for (int i = i0 + t; i < S; i += kTileThreads) xs[tile_at<XT>(i)] = i < have ? xt[i] : first;
     __syncthreads();
