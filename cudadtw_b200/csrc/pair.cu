@@ -379,6 +379,11 @@ int launch_pair_fwd(cdtw_handle h, const float* zq, const float* zs, int64_t n, 
     size_t shared_rec;
     const bool shared = pair_shared_record(L, G, C, &a.recb, &a.logb, &shared_rec);
     const int dm = !rows ? 0 : shared ? 2 : mode == 1 ? 5 : 1;
+    if (shared) {  // room in front of each record (the bank stride kept)
+        const int pad = (int)round_up(shared_pad<1>(G), 128);
+        a.recb += pad;
+        shared_rec += (size_t)groups_per_block * pad;
+    }
     if (dm == 5) {
         a.ckpt = (float*)dirs;
         a.seg = thin_seg(C);

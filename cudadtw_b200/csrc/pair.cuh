@@ -329,6 +329,13 @@ __device__ __forceinline__ void runs_from_moves(const uint8_t* mlog, int nm, int
     }
 }
 
+// Bytes in front of a shared-memory record: two anti-diagonals and an element,
+// which the walk's loads may touch.
+template <int C>
+__host__ __device__ constexpr int shared_pad(int G) {
+    return ((2 * G + 1) * (int)sizeof(DirT<C>) + 3) / 4 * 4;
+}
+
 // One walker move from slot c of lane lw on anti-diagonal kw (parity e) by
 // code b: diagonal keeps the slot, up (d + 1) / left (d - 1) move to slot
 // c + e / c + e - 1 of the other parity.  Branch-free (the walkers of a warp
@@ -362,20 +369,25 @@ __device__ __forceinline__ void walk_shared(const PairArgs& a, unsigned char* sm
     if (l == 0 && live) {
         r16[2 * (L - 1) + 1] = (uint16_t)(L - 1);
         c16[2 * (L - 1) + 1] = (uint16_t)(L - 1);
-        int kw = K - 1, e = e0, lw = porg / C, c = porg - lw * C;
-        uint32_t cur = rec[(size_t)kw * G + lw];
-        // every move lowers kw, so at most K moves (the log holds K bytes)
-        while (kw >= 0 && (unsigned)lw < (unsigned)G) {
-            const int r1 = max(kw - 1, 0), r2 = max(kw - 2, 0);
-            const uint32_t n2 = rec[r2 * G + lw];
-            const uint32_t n1 = rec[r1 * G + lw];
-            const uint32_t n1m = rec[r1 * G + max(lw - 1, 0)];
-            const uint32_t n1p = rec[r1 * G + min(lw + 1, G - 1)];
+        int e = e0, lw = porg / C, c = porg - lw * C;
+        int at = (K - 1) * G + lw;  // element of the walker's anti-diagonal and lane
+        uint32_t cur = rec[at];
+        // every move lowers the anti-diagonal, so at most K moves (the log holds
+        // K bytes); the loads before anti-diagonal 0 fall into the record's pad
+        while (at >= 0 && (unsigned)lw < (unsigned)G) {
+            const DT* below = rec + at - G;
+            const uint32_t n2 = below[-G], n1 = below[0], n1m = below[-1], n1p = below[1];
             const uint32_t b = (cur >> (2 * c)) & 3u;
             mlog[nm++] = (uint8_t)b;
-            const int lw0 = lw;
-            walk_move<C>(b, kw, e, lw, c);
-            cur = (b & 1u) ? n2 : (lw > lw0 ? n1p : (lw < lw0 ? n1m : n1));
+            const bool dg = b & 1u;
+            const int cn = c + (dg ? 0 : (b ? e : e - 1));  // up keeps or raises the slot
+            const bool hi = cn >= C, lo = cn < 0;
+            const int dl = hi ? 1 : (lo ? -1 : 0);
+            at += dg ? -2 * G : dl - G;
+            c = cn + (hi ? -C : (lo ? C : 0));
+            lw += dl;
+            e ^= dg ? 0 : 1;
+            cur = dg ? n2 : (hi ? n1p : (lo ? n1m : n1));
         }
     }
     nm = __shfl_sync(kFull, nm, 0, G);
@@ -568,7 +580,7 @@ __global__ void __launch_bounds__(kPairThreads, 4) pair_fwd_kernel(const PairArg
     const int porg = W >> 1;  // slot of d = 0 on every anti-diagonal of parity e0
     PairLane<C> st;
     uint32_t* drow = DM == 1   ? a.dirs + (size_t)pr * a.dstride
-                     : DM == 2 ? (uint32_t*)(smem + (size_t)gib * a.recb)
+                     : DM == 2 ? (uint32_t*)(smem + (size_t)gib * a.recb + shared_pad<C>(G))
                                : nullptr;
     int k = pair_begin<C, EU, DM>(st, sq, ss, drow, L, W, G, l, K, live);
     NextCkpt nc{nullptr, K};
