@@ -136,12 +136,11 @@ int launch_pair_znorm(cdtw_handle h, const float* q, const float* s, int64_t n, 
 // path record) lane groups of 32 with the fewest cells per lane -- the
 // shortest step, for a handful of pairs.  store: a path record keeps direction
 // bits in dirs; otherwise dirs holds checkpoints where that is the faster way
-// (pair_auto_mode).
+// (pair_auto_mode; h->last_pair_recompute is set then).
 int launch_pair_fwd(cdtw_handle h, const float* zq, const float* zs, int64_t n, int L, int W,
                     bool euclid, float* D, uint32_t* dirs, uint32_t* rows, uint32_t* cols,
                     int64_t qstride = -1, const int* gate = nullptr, int gate_max = 0,
                     int gate_min = -1, bool wide = false, bool store = false);
-int pair_auto_mode(int L, int W);
 // Checkpointed path record (memory: pair_ckpt_floats per pair instead of the
 // direction scratch); pair_ckpt_floats is 0 where the mode does not apply.
 size_t pair_ckpt_floats(int L, int W);

@@ -310,12 +310,16 @@ static size_t pair_thin_floats(int L, int W, int G, int C) {
 // bits and 251 with thin checkpoints, 512 of 2048, W = 409, 1460 / 483 and 612
 // with wide ones.  Thin ones need their floats to fit the bits' scratch, which
 // leaves out bands within 1/16 of a power-of-two group's full width and
-// W >= 480; wide ones serve those of W >= 128.
-int pair_auto_mode(int L, int W) {
+// W >= 480; wide ones serve those of W >= 128.  Bands that a walk's 32 slots
+// hold whole are walked again in full, a warp a pair: bits are the faster once
+// the pairs fill the chip (14 warps an SM; L = 300, W = 30, bits / checkpoints
+// 122 / 153 us at 4000 pairs, W = 15 128 / 96 at 1000 and 134 / 143 at 4000).
+static int pair_auto_mode(cdtw_handle h, int64_t n, int L, int W) {
     int G, C;
     pair_shape(L, W, &G, &C);
     const size_t words = pair_dirs_words(L, W);
     if (words == 0 || C < 2 || C > 16) return 0;
+    if (W + 1 <= 32 && n > 14 * (int64_t)h->sm_count) return 0;
     if (thin_seg(C) <= kThinSeg && pair_thin_floats(L, W, G, C) <= words) return 1;
     return C > kCorridorC && pair_ckpt_floats(L, W) <= words ? 2 : 0;
 }
@@ -336,7 +340,8 @@ int launch_pair_fwd(cdtw_handle h, const float* zq, const float* zs, int64_t n, 
     int G, C;
     pair_shape(L, W, &G, &C);
     if (C > 16) return set_error(h, CDTW_EUNSUPPORTED, "pair band W=%d exceeds 511", W);
-    const int mode = rows && cols && dirs && !store ? pair_auto_mode(L, W) : 0;
+    const int mode = rows && cols && dirs && !store ? pair_auto_mode(h, n, L, W) : 0;
+    if (mode) h->last_pair_recompute = 1;
     if (mode == 2)
         return launch_pair_fwd_ckpt(h, zq, zs, n, L, W, euclid, D, (float*)dirs, rows, cols);
     if (!rows && wide) {

@@ -42,3 +42,21 @@ def test_path_from_checkpoints_equals_stored_directions(L, W, n, kind, metric):
     for mode in (None, "recompute"):
         assert torch.equal(got[mode][0], got["store"][0])
         assert torch.equal(got[mode][1], got["store"][1])
+
+
+@pytest.mark.parametrize("W", [15, 31, 32])
+@pytest.mark.parametrize("over", [0, 1])
+def test_default_path_at_the_chip_filling_count(W, over):
+    # narrow bands (W + 1 <= 32 slots) keep direction bits above 14 pairs an SM
+    from cudadtw_b200 import Handle
+    n = 14 * torch.cuda.get_device_properties(0).multi_processor_count + over
+    q, s = _series("walk", n, 290, W)
+    got = {}
+    with Handle(0) as h:
+        for mode in (None, "recompute", "store"):
+            path = torch.zeros(h.pair_path_bytes(n, 290), dtype=torch.uint8, device="cuda")
+            D = h.pair_fwd(q, s, W, path=path, mode=mode)
+            got[mode] = (D.cpu(), path.cpu())
+    for mode in (None, "recompute"):
+        assert torch.equal(got[mode][0], got["store"][0])
+        assert torch.equal(got[mode][1], got["store"][1])
