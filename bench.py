@@ -332,7 +332,7 @@ def subresults(h, dev, peak=None) -> dict:
       walks) and its L=2048/W=409 variant: forward (D only), forward with the
       path record, backward, and their ratio; CUDA-graph replays, device time.
     * wide_band_all_windows: all-windows cDTW of 2^18 windows at M=1024 for
-      W = 102, 204, 409 (the lane-group kernel).
+      W = 102 (register band), 204 and 409 (lane groups).
     """
     import torch
     from cudadtw_b200 import synth
@@ -568,7 +568,7 @@ def subresults(h, dev, peak=None) -> dict:
         h.gpu_cdtw(dx, avg, std)  # warm-up
         t, _ = dev_time_median(lambda: h.gpu_cdtw(dx, avg, std))
         g = (1 << 18) * cells(1024, W) / t / 1e9
-        wide[f"W{W}"] = {"ms": t * 1e3, "gcups": g, "variant": "lane group",
+        wide[f"W{W}"] = {"ms": t * 1e3, "gcups": g, "variant": "register band" if W <= 106 else "lane group",
                          "frac_of_measured_cell_rate": g / (peak / 1e9) if peak else None}
     out["wide_band_all_windows"] = {"stream": "metal 2^18 windows", "M": 1024, "bands": wide}
     del dx
