@@ -5,9 +5,10 @@
 // stats.cuh:85-142) and then takes the variance in FP32 (stats.cuh:49), which
 // loses the variance of level-shifted signals.  Here one kernel reads the
 // stream once per tile of kTileWindows windows: FP64 sums of (x-c) and
-// (x-c)^2, c the tile's first sample, per chunk of eight samples, a block scan
-// over the chunks, and per thread eight windows slid from the difference of
-// two prefixes.  Output per window: mean (FP64) and sigma (FP32), 12 bytes.
+// (x-c)^2 per chunk of 16 samples, c the chunk's first one, joined over blocks
+// of two, four, ... chunks, and per thread 16 windows slid from one that is
+// put together from such blocks.  Output per window: mean (FP64) and sigma
+// (FP32), 12 bytes.
 #include "common.cuh"
 
 #include <algorithm>
@@ -122,7 +123,8 @@ avg_std_long_kernel(const XT* __restrict__ x, int64_t N, int M, double* __restri
 // Deviation of a positive variance.  For the FP32 result: an FP32 estimate
 // (s0 = v * rsqrt(v)) and one Heron step whose residual v - s0^2 is taken in
 // FP64, so the result is the FP64 root rounded to FP32 but for ties within
-// 1e-7 ulp, at a fraction of the FP64 square root's instructions.
+// 1e-6 ulp (an estimate within 2e-7 leaves 4e-14 of the root), at a fraction of
+// the FP64 square root's instructions.
 template <bool INV>
 __device__ __forceinline__ double std_of(double var, double) {
     return var > 0.0 ? (INV ? rsqrt(var) : sqrt(var)) : 1.0;
@@ -142,27 +144,32 @@ __device__ __forceinline__ float std_of(double var, float) {
 // One block per tile of kTileWindows windows, kTileR = 16 consecutive windows
 // per thread.  The tile's kTileWindows + M samples are staged in shared memory
 // with one 16-byte pad per 16 samples, so a warp's 16-byte accesses (lanes 16
-// samples apart) fall on all banks; chunk c holds samples 16c .. 16c+15.  The
-// sums of a thread's first window are the prefix at 16t + M (the chunk prefix
-// plus M mod 16 samples) less the prefix at 16t; the others follow by sliding,
-// the leaving samples still in registers.  Results go out through shared
-// memory in whole lines.
+// samples apart) fall on all banks; chunk c holds samples 16c .. 16c+15.  Blocks
+// of 2^k chunks, from every chunk on, hold their sums about their first sample;
+// a thread's first window is the sum of the blocks of M / 16's binary digits and
+// the M mod 16 samples behind them, moved to its own first sample; the others
+// follow by sliding, the leaving samples still in registers.  Results go out
+// through shared memory in whole lines.
 //
-// Where the variance is below 2^-22 of the prefix it was taken from (over M:
-// 2^30 units in the prefix's last place; flat runs, a level shift inside the
-// tile) the difference of prefixes may have lost it, and a NaN or Inf sample
-// leaves the prefixes behind it without a value: such windows are summed again
-// about their own first sample, so a constant window has variance exactly 0
-// (sigma 1) wherever it lies and a bad sample spoils the windows that hold it
-// only.
+// No sum holds samples outside the thread's 16 windows, so nothing else in the
+// tile (a level shift, a flat run, a bad sample) touches them: a constant window
+// has variance exactly 0 (sigma 1).  What is left is the slide: where the
+// variance is below kLost of the second moment it came from (a large sample that
+// left), or a NaN or Inf sample left, the windows behind are summed again, the
+// first by the warp in two passes, the next slid from it.  For M < 16 a sample
+// may enter and leave within the 16 windows, so there the moment is that of all
+// their samples, and such windows are summed one by one.
+//
+// Precision: with the sums as differences of prefixes over the tile, FP64
+// sigmas were off by up to 9e-13 (ECG-like, M = 64; 8e-14 by the run of 512
+// windows of avg_std_long_kernel), now 5e-14.
 //
 // Bound: HBM (16 bytes a window, 82 us at 2^25 windows and 6546 GB/s) if the
-// latencies of a block's phases were hidden; 72 instructions a window, 24
-// warps per SM.  Six blocks per SM (80 registers, 100 bytes spilled) measured
-// best (5 / 6 / 7: 146 / 144 / 144 us at 2^25 windows, M = 512), the samples
-// copied asynchronously (156 us through registers).  2^20 windows, M = 128: 10
-// us.  Before (a warp per 2048 windows, scans of 32 windows a round): 196 and
-// 22 us, the latter the latency of its serial rounds.
+// latencies of a block's phases were hidden.  Six blocks per SM (80 registers,
+// 84 bytes spilled) measured best at 2^25 windows, M = 512: 144 us, five 155;
+// for FP64 sigmas four (no spills).  2^20 windows, M = 128: 10 us; a warp per
+// 2048 windows and scans of 32 windows a round took 196 and 22.  A NaN every
+// 3000 samples, M = 2000, 2^20 windows: 19 us, 12 without them.
 constexpr int kTileThreads = 128;
 constexpr int kTileR = 16;                                // windows per thread, samples per chunk
 constexpr int kTileWindows = kTileThreads * kTileR;       // 2048
@@ -177,7 +184,7 @@ __host__ __device__ constexpr int tile_at(int i) {
 template <class XT, class ST>
 size_t tile_smem(int M) {
     const int S = (int)round_up(kTileWindows + M, kTileR), NC = S / kTileR;
-    const size_t in = sizeof(XT) * (size_t)tile_at<XT>(S) + 2 * sizeof(double) * (size_t)NC;
+    const size_t in = sizeof(XT) * (size_t)tile_at<XT>(S) + (2 * sizeof(double2) + sizeof(XT)) * (size_t)NC;
     return std::max(in, sizeof(double) * (size_t)tile_at<double>(kTileWindows));
 }
 
@@ -248,18 +255,29 @@ __device__ __forceinline__ void tile_entering(const double* xs, int t, int M, do
     for (int k = 0; k < 16; ++k) v[k] = b1 ? y[k + 1] : y[k];
 }
 
-// Mean and variance of the window at tile sample i0, about its first sample.
-template <class XT>
-__device__ __noinline__ double2 tile_window(const XT* xs, int i0, int M) {
-    const double f = (double)xs[tile_at<XT>(i0)], invM = 1.0 / (double)M;
-    double a1 = 0.0, a2 = 0.0;
-    for (int k = 1; k < M; ++k) {
-        const double d = (double)xs[tile_at<XT>(i0 + k)] - f;
-        a1 += d;
-        a2 = fma(d, d, a2);
+// Mean and variance of the window x[0 .. M) in two passes, the samples from
+// `lane` on, `lanes` apart (1: by one thread; 32: by a warp, all of whose lanes
+// get both).
+template <int lanes, class XT>
+__device__ __noinline__ double2 window_stats(const XT* __restrict__ x, int M, int lane) {
+    const double f = (double)x[0], invM = 1.0 / (double)M;
+    double m = 0.0, v = 0.0;
+    for (int k = lane; k < M; k += lanes) m += (double)x[k] - f;
+    m = f + (lanes == 32 ? warp_sum(m) : m) * invM;
+    for (int k = lane; k < M; k += lanes) {
+        const double d = (double)x[k] - m;
+        v = fma(d, d, v);
     }
-    a1 *= invM;
-    return make_double2(f + a1, fma(-a1, a1, a2 * invM));
+    return make_double2(m, (lanes == 32 ? warp_sum(v) : v) * invM);
+}
+
+// The sums (s1, s2) of n samples about g as part of sums about g - dl, added
+// to (a1, a2).
+__device__ __forceinline__ void tile_add(double& a1, double& a2, const double2& s, double dl,
+                                         double n) {
+    const double e = n * dl;
+    a1 += s.x + e;
+    a2 += fma(dl, fma(2.0, s.x, e), s.y);
 }
 
 // The tile's n results, 16 of them in each thread's v, to out through z (16-byte
@@ -283,23 +301,23 @@ __device__ __forceinline__ void tile_out(T* z, const T (&v)[kTileR], T* __restri
 
 // mu may be null (not wanted); INV: sigma takes 1 / sigma.
 template <class XT, class ST, bool INV>
-__global__ void __launch_bounds__(kTileThreads, 6)
+__global__ void __launch_bounds__(kTileThreads, sizeof(ST) == 8 ? 4 : 6)
 avg_std_kernel(const XT* __restrict__ x, int64_t N, int M, double* __restrict__ mu,
                ST* __restrict__ sigma) {
     extern __shared__ __align__(16) unsigned char tsm[];
-    constexpr int kWarps = kTileThreads / 32;
     constexpr int V = 16 / (int)sizeof(XT);  // samples of a 16-byte vector
-    __shared__ double tot[2][kWarps];
+    // variance, of the second moment it is left from, below which it is taken again
+    constexpr unsigned kAll = (1u << kTileR) - 1u;
+    constexpr double kLost = sizeof(ST) == 8 ? 0x1p-10 : 0x1p-22;
     const int64_t Nw = N - M + 1;
     const int64_t t0 = (int64_t)blockIdx.x * kTileWindows;
-    const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+    const int t = threadIdx.x, lane = t & 31;
     const int S = (kTileWindows + M + kTileR - 1) / kTileR * kTileR, NC = S / kTileR;
     XT* xs = (XT*)tsm;
-    double* C1 = (double*)(xs + tile_at<XT>(S));
-    double* C2 = C1 + NC;
+    double2* cur = (double2*)(xs + tile_at<XT>(S));  // sums of blocks of chunks from each chunk on
+    double2* nxt = cur + NC;
+    XT* fs = (XT*)(nxt + NC);  // first sample of every chunk
     const XT* __restrict__ xt = x + t0;
-    const XT first = xt[0];
-    const double c = (double)first;
     // samples past the stream enter windows that are not stored only
     const int have = (int)min((int64_t)S, N - t0);
     int i0 = 0;
@@ -312,106 +330,130 @@ avg_std_kernel(const XT* __restrict__ x, int64_t N, int M, double* __restrict__ 
                          : "memory");
         asm volatile("cp.async.wait_all;" ::: "memory");
     }
-    for (int i = i0 + t; i < S; i += kTileThreads) xs[tile_at<XT>(i)] = i < have ? xt[i] : first;
+    for (int i = i0 + t; i < S; i += kTileThreads) xs[tile_at<XT>(i)] = i < have ? xt[i] : XT(0);
     __syncthreads();
-    // chunk sums and their exclusive prefix, kTileThreads chunks a round
-    double v[kTileR];  // the thread's own chunk, about c
-    double base1 = 0.0, base2 = 0.0;
-    for (int r0 = 0; r0 < NC; r0 += kTileThreads) {
-        if (r0) __syncthreads();  // the previous round's totals are read
-        const int ch = r0 + t;
-        double e1 = 0.0, e2 = 0.0;
-        if (r0 + 32 * wid < NC) {  // whole warps
-            double a1 = 0.0, a2 = 0.0;
-            XT xv[kTileR];
-            tile_load16(xs + (kTileR + V) * min(ch, NC - 1), xv);
-            if (ch < NC) {
+    // sums of every chunk about its first sample
+    double v[kTileR], c = 0.0;  // the thread's own chunk, about c
+    unsigned again = 0;         // windows to be summed again
+    for (int ch = t; ch < NC; ch += kTileThreads) {
+        XT xv[kTileR];
+        tile_load16(xs + (kTileR + V) * ch, xv);
+        const double f = (double)xv[0];
+        double a1 = 0.0, a2 = 0.0;
 #pragma unroll
-                for (int k = 0; k < kTileR; ++k) {
-                    const double d = (double)xv[k] - c;
-                    if (r0 == 0) v[k] = d;
-                    a1 += d;
-                    a2 = fma(d, d, a2);
-                }
-            }
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const double u1 = __shfl_up_sync(0xffffffffu, a1, o);
-                const double u2 = __shfl_up_sync(0xffffffffu, a2, o);
-                if (lane >= o) {
-                    a1 += u1;
-                    a2 += u2;
-                }
-            }
-            e1 = __shfl_up_sync(0xffffffffu, a1, 1);
-            e2 = __shfl_up_sync(0xffffffffu, a2, 1);
-            if (lane == 0) e1 = e2 = 0.0;
-            if (lane == 31) {
-                tot[0][wid] = a1;
-                tot[1][wid] = a2;
-            }
-        } else if (lane == 31) {
-            tot[0][wid] = tot[1][wid] = 0.0;
+        for (int k = 0; k < kTileR; ++k) {
+            const double d = (double)xv[k] - f;
+            if (ch == t) v[k] = d;
+            a1 += d;
+            a2 = fma(d, d, a2);
         }
+        if (ch == t) {
+            c = f;
+            if (!(a2 < (double)CDTW_INF)) {  // bad samples spoil the slide behind them
+                again = kAll;
+                for (int k = 0; k < kTileR; ++k)
+                    if (!(fabs((double)xs[(kTileR + V) * t + k]) < (double)CDTW_INF))
+                        again = kAll & (kAll << (k + 1));
+            }
+        }
+        cur[ch] = make_double2(a1, a2);
+        fs[ch] = xv[0];
+    }
+    // sums of the thread's first window about its first sample: its n chunks as
+    // blocks of the powers of two in n, then the samples of a part of a chunk
+    const int n = M / kTileR, rest = M % kTileR;
+    double w1 = 0.0, w2 = 0.0;
+    for (int b = 1, len = 0; b <= n; b *= 2) {  // cur: blocks of b chunks
         __syncthreads();
-        double b1 = base1, b2 = base2;
-#pragma unroll
-        for (int w = 0; w < kWarps; ++w) {
-            const double u1 = tot[0][w], u2 = tot[1][w];
-            b1 += w < wid ? u1 : 0.0;
-            b2 += w < wid ? u2 : 0.0;
-            base1 += u1;
-            base2 += u2;
+        if (n & b) {
+            tile_add(w1, w2, cur[t + len], (double)fs[t + len] - c, 16.0 * b);
+            len += b;
         }
-        if (ch < NC) {
-            C1[ch] = b1 + e1;
-            C2[ch] = b2 + e2;
+        if (2 * b <= n) {
+            // from here on chunks t + (n mod 2b) and further are looked at
+            for (int ch = t + (n & (2 * b - 1)); ch < kTileThreads + n - 2 * b;
+                 ch += kTileThreads) {
+                double2 a = cur[ch];
+                tile_add(a.x, a.y, cur[ch + b], (double)fs[ch + b] - (double)fs[ch], 16.0 * b);
+                nxt[ch] = a;
+            }
+            double2* const swap = cur;
+            cur = nxt;
+            nxt = swap;
         }
     }
-    __syncthreads();
-    // sums of the thread's first window
-    const int e = kTileR * t + M, ce = e / kTileR, rest = e % kTileR;
-    double w1 = C1[ce], w2 = C2[ce];
     for (int k = 0; k < rest; ++k) {
-        const double d = (double)xs[(kTileR + V) * ce + k] - c;
+        const double d = (double)xs[(kTileR + V) * (t + n) + k] - c;
         w1 += d;
         w2 = fma(d, d, w2);
     }
     const double invM = 1.0 / (double)M;
-    const double lost = w2 * invM * 0x1p-22;
-    w1 -= C1[t];
-    w2 -= C2[t];
+    double most = w2;  // the second moment that the slide's sums may have held
+    if (n == 0) {      // a sample may enter and leave again: all of them
+        for (int k = M; k < M + kTileR; ++k) {
+            const double d = (double)xs[tile_at<XT>(kTileR * t + k)] - c;
+            most = fma(d, d, most);
+        }
+        again = most < (double)CDTW_INF ? 0u : kAll;
+    }
+    const double lost = most * invM * kLost;
     XT in[kTileR];
     tile_entering(xs, t, M, in);
     double om[kTileR];
     ST os[kTileR];
-    unsigned again = 0;  // windows to be summed again
 #pragma unroll
     for (int r = 0; r < kTileR; ++r) {
         const double m1 = w1 * invM;
         const double var = fma(-m1, m1, w2 * invM);
         om[r] = c + m1;
         os[r] = std_of<INV>(var, ST());
-        again |= var >= lost ? 0u : 1u << r;
+        again |= var < lost ? 1u << r : 0u;
         const double vin = (double)in[r] - c, d = vin - v[r];
         w1 += d;
         w2 = fma(d, vin + v[r], w2);
     }
-    if (again) {
-#pragma unroll
-        for (int r = 0; r < kTileR; ++r) {
-            if ((again >> r & 1u) && t0 + kTileR * t + r < Nw) {
-                const double2 q = tile_window(xs, kTileR * t + r, M);
-                om[r] = q.x;
-                os[r] = std_of<INV>(q.y, ST());
-            }
-        }
-    }
-    // the samples and prefixes make room for the sigmas, these for the means
+    // the samples and sums make room for the sigmas, these for the means
     tile_out(reinterpret_cast<ST*>(tsm), os, sigma + t0, (int)min((int64_t)kTileWindows, Nw - t0));
     if (mu)
         tile_out(reinterpret_cast<double*>(tsm), om, mu + t0,
                  (int)min((int64_t)kTileWindows, Nw - t0));
+    // the windows to be summed again, from the stream
+    const int left = (int)min(Nw - t0 - kTileR * t, (int64_t)kTileR);  // the thread's windows
+    again &= left <= 0 ? 0u : kAll >> (kTileR - left);
+    if (!__syncthreads_or((int)again)) return;
+    auto put = [&](int r, double m, double var) {
+        if (mu) mu[t0 + kTileR * t + r] = m;
+        sigma[t0 + kTileR * t + r] = std_of<INV>(var, ST());
+    };
+    if (n == 0) {
+        for (; again; again &= again - 1) {
+            const int r = __ffs(again) - 1;
+            const double2 q = window_stats<1>(xt + kTileR * t + r, M, 0);
+            put(r, q.x, q.y);
+        }
+        return;
+    }
+    // a lane's first one by the warp; the lane slides on from there
+    while (const unsigned need = __ballot_sync(0xffffffffu, again != 0)) {
+        const int src = __ffs(need) - 1;
+        const int r0 = __ffs(__shfl_sync(0xffffffffu, again, src)) - 1;
+        const double2 q = window_stats<32>(xt + kTileR * (t - lane + src) + r0, M, lane);
+        if (lane == src) {
+            again = 0;
+            w1 = 0.0;
+            w2 = q.y * (double)M;
+            const XT* xw = xt + kTileR * t;
+            for (int r = r0;; ++r) {
+                const double m1 = w1 * invM, var = fma(-m1, m1, w2 * invM);
+                put(r, q.x + m1, var);
+                if (var < q.y * kLost) again |= 1u << r;
+                if (r + 1 >= left) break;
+                const double vin = (double)xw[r + M] - q.x, out = (double)xw[r] - q.x;
+                w1 += vin - out;
+                w2 = fma(vin - out, vin + out, w2);
+            }
+        }
+    }
 }
 
 // One block prepares the query pack: FP64 two-pass z-normalisation (the
