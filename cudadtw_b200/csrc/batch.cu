@@ -250,9 +250,7 @@ int batch_grid(cdtw_handle h, bool euclid, size_t smem, int* blocks) {
     int best = 1 << 30;
     for (int i = 0; i < 3; ++i) {
         const size_t sm = (i == 2) ? 0 : smem;
-        if (sm > 48 * 1024)
-            CDTW_CUDA(h, cudaFuncSetAttribute(ks[i], cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              (int)sm));
+        CDTW_TRY(allow_smem(h, ks[i], sm));
         int per = 0;
         CDTW_CUDA(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, ks[i], kBatchThreads, sm));
         best = std::min(best, std::max(per, 1));

@@ -33,9 +33,7 @@ const BatchRegKernels& batch_reg_kernels() {
 int batch_reg_prepare(cdtw_handle h, int W, bool euclid, size_t smem, int* blocks) {
     if (W < 0 || W > kMaxBatchRegW) return set_error(h, CDTW_EINVAL, "register band %d out of range", W);
     const void* k = (const void*)(euclid ? batch_reg_kernels().eu[W] : batch_reg_kernels().mh[W]);
-    if (smem > 48 * 1024)
-        CDTW_CUDA(h, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)smem));
+    CDTW_TRY(allow_smem(h, k, smem));
     int per = 0;
     CDTW_CUDA(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, kBatchThreads, smem));
     *blocks = std::max(per, 1) * h->sm_count;

@@ -386,7 +386,7 @@ int launch_stream_envelope(cdtw_handle h, const float* x, int64_t N, int W, floa
     const int T = std::max(1, std::min(std::max(2048, 2 * W), kEnvSmemFloats / arrays - 2 * W));
     const size_t smem = (size_t)arrays * (T + 2 * W) * sizeof(float);
     const void* k = ping ? (const void*)env_window_kernel<true> : (const void*)env_window_kernel<false>;
-    CDTW_CUDA(h, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    CDTW_TRY(allow_smem(h, k, smem));
     int per_sm = 0;
     CDTW_CUDA(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kEnvThreads, smem));
     const unsigned grid = (unsigned)std::max<int64_t>(

@@ -16,6 +16,20 @@ int set_error(cdtw_handle h, int status, const char* fmt, ...) {
     return status;
 }
 
+int allow_smem(cdtw_handle h, const void* k, size_t smem) {
+    if (smem <= 32 * 1024) return CDTW_OK;  // within the limit of every kernel as it is
+    const void*& slot = h->smem_set[((uintptr_t)k >> 4) % 61];
+    if (slot == k) return CDTW_OK;
+    int all = 0;
+    CDTW_CUDA(h, cudaDeviceGetAttribute(&all, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device));
+    cudaFuncAttributes fa;
+    CDTW_CUDA(h, cudaFuncGetAttributes(&fa, k));
+    CDTW_CUDA(h, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      all - (int)fa.sharedSizeBytes));
+    slot = k;
+    return CDTW_OK;
+}
+
 int check_cuda(cdtw_handle h, cudaError_t e, const char* what) {
     if (e == cudaSuccess) return CDTW_OK;
     if (e == cudaErrorMemoryAllocation) {

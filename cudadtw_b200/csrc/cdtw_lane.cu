@@ -175,8 +175,7 @@ int launch_cdtw_lane(cdtw_handle h, const float* x, int64_t N, const double* mu,
     a.out = out;
     const LaneKernel k = euclid ? lane_kernels().eu[B] : lane_kernels().mh[B];
     const size_t smem = lane_smem(h->q);
-    CDTW_CUDA(h, cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)smem));
+    CDTW_TRY(allow_smem(h, (const void*)k, smem));
     const int64_t units = div_up(L, 2);
     const int64_t per_block = kLaneThreads / G;
     const int64_t blocks = div_up(units, per_block);
@@ -203,8 +202,7 @@ int launch_cdtw_lane_search(cdtw_handle h, const float* x, int64_t N, const doub
     a.sink = sink;
     const LaneKernel k = euclid ? lane_kernels().seu[B] : lane_kernels().smh[B];
     const size_t smem = lane_smem(h->q);
-    CDTW_CUDA(h, cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)smem));
+    CDTW_TRY(allow_smem(h, (const void*)k, smem));
     int per_sm = 0;
     CDTW_CUDA(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)k,
                                                                kLaneThreads, smem));

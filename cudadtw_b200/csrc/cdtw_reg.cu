@@ -97,8 +97,7 @@ int launch_cdtw_search(cdtw_handle h, const float* x, int64_t N, const double* m
     RegSearchKernel k = euclid ? reg_kernels().seu[q.W] : reg_kernels().smh[q.W];
     const int lq4 = q.lq / 4;
     const size_t smem = (size_t)q.lq * sizeof(float) + (size_t)reg_env_len(q.M) * sizeof(float2);
-    CDTW_CUDA(h, cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)smem));
+    CDTW_TRY(allow_smem(h, (const void*)k, smem));
     int per_sm = 0;
     CDTW_CUDA(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)k, kRegBlock,
                                                                smem));
@@ -130,9 +129,7 @@ int launch_cdtw_windows(cdtw_handle h, const float* x, int64_t N, const double* 
     const int lq4 = q.lq / 4;
     const size_t smem = (size_t)q.lq * sizeof(float);
     auto prepare = [&](const void* k) -> int {
-        if (smem > 48 * 1024)
-            CDTW_CUDA(h, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              (int)smem));
+        CDTW_TRY(allow_smem(h, k, smem));
         return CDTW_OK;
     };
     if (!idx && L == Nw) {

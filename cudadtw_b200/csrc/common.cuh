@@ -95,12 +95,20 @@ struct cdtw_handle_s {
     cudaStream_t xfer[3] = {nullptr, nullptr, nullptr};
     cudaEvent_t xev[3 * 16 + 1] = {};
     bool xready = false;
+    // kernels whose shared-memory limit this handle has raised (allow_smem)
+    const void* smem_set[64] = {};
     char err[512] = {0};
 };
 
 namespace cdtw {
 
 int set_error(cdtw_handle h, int status, const char* fmt, ...);
+// Before a launch of kernel k with smem bytes of dynamic shared memory, or a
+// question about its occupancy: raises the kernel's limit to all that the device
+// has.  The limit belongs to the device, not to the handle: set to what each
+// launch needs, a second thread's smaller size came between the first one's
+// setting and its launch, which then failed.
+int allow_smem(cdtw_handle h, const void* k, size_t smem);
 // Bytes of a query pack for (M, W); with q and base, points q's arrays into
 // base (device memory of at least that many bytes).
 size_t query_pack_layout(int M, int W, QueryPack* q, char* base);

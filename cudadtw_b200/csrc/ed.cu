@@ -226,8 +226,7 @@ int launch_ed(cdtw_handle h, const double* x, int64_t N, const double* zq, int M
               const double* rs, double* out) {
     const int64_t Nw = N - M + 1;
     const size_t smem = 2 * kEdStage * sizeof(double);
-    CDTW_CUDA(h, cudaFuncSetAttribute((const void*)ed_kernel,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    CDTW_TRY(allow_smem(h, (const void*)ed_kernel, smem));
     int per_sm = 0;
     CDTW_CUDA(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)ed_kernel,
                                                                kEdThreads, smem));

@@ -352,12 +352,9 @@ int launch_ldtw_ref(cdtw_handle h, const float* x, int64_t N, bool euclid, bool 
     const unsigned blocks = (unsigned)div_up(Nw, kRefWin);
     auto k = euclid ? (znorm ? ldtw_ref_kernel<true, true> : ldtw_ref_kernel<true, false>)
                     : (znorm ? ldtw_ref_kernel<false, true> : ldtw_ref_kernel<false, false>);
-    // the query pairs and the block's samples: above 48 KB from M = 4010
+    // the query pairs and the block's samples
     const size_t smem = sizeof(float) * (size_t)(3 * q.M + kRefWin + 5);
-    if (smem > 48 * 1024)
-        CDTW_CUDA(h, cudaFuncSetAttribute((const void*)k,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)smem));
+    CDTW_TRY(allow_smem(h, (const void*)k, smem));
     k<<<blocks, kRefWin, smem, h->stream>>>(x, zq, q.M, q.W, Nw, out);
     CDTW_LAUNCH(h, "ldtw_ref_kernel");
     return CDTW_OK;

@@ -405,8 +405,7 @@ int launch_pair_fwd(cdtw_handle h, const float* zq, const float* zs, int64_t n, 
     const int64_t blocks = div_up(n, groups_per_block);
     if (blocks > INT32_MAX) return set_error(h, CDTW_EINVAL, "too many pairs");
     const PairFwdK k = fwd_kernel(C, euclid, dm);
-    CDTW_CUDA(h, cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)smem));
+    CDTW_TRY(allow_smem(h, (const void*)k, smem));
     k<<<(int)blocks, threads, smem, h->stream>>>(a);
     CDTW_LAUNCH(h, "pair_fwd_kernel");
     if (dm == 5) {
@@ -473,8 +472,7 @@ int launch_pair_fwd_ckpt(cdtw_handle h, const float* zq, const float* zs, int64_
                   : (euclid ? pair_corridor_kernel<kCorridorC, true>
                             : pair_corridor_kernel<kCorridorC, false>);
     const size_t smem = (size_t)groups_per_block * (size_t)(a.recb + a.logb);
-    CDTW_CUDA(h, cudaFuncSetAttribute((const void*)kw, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)smem));
+    CDTW_TRY(allow_smem(h, (const void*)kw, smem));
     kw<<<(int)blocks, threads, smem, h->stream>>>(a);
     CDTW_LAUNCH(h, corridor ? "pair_corridor_kernel" : "pair_ckpt_walk_kernel");
     return CDTW_OK;
@@ -495,8 +493,7 @@ int launch_pair_bwd(cdtw_handle h, const float* q, const float* s, int64_t n, in
     if (blocks > INT32_MAX) return set_error(h, CDTW_EINVAL, "too many pairs");
     auto k = euclid ? (block ? pair_bwd_kernel<true, true> : pair_bwd_kernel<true, false>)
                     : (block ? pair_bwd_kernel<false, true> : pair_bwd_kernel<false, false>);
-    CDTW_CUDA(h, cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)smem));
+    CDTW_TRY(allow_smem(h, (const void*)k, smem));
     k<<<(unsigned)blocks, block ? kBwdThreads : nw * 32, smem, h->stream>>>(q, s, n, L, hdr, rows,
                                                                            cols, dD, dq, ds);
     CDTW_LAUNCH(h, "pair_bwd_kernel");

@@ -667,8 +667,7 @@ int launch_keogh(cdtw_handle h, const float* x, int64_t N, const double* mu, con
         }
     }
     const size_t smem = (size_t)wpb * per_warp;
-    CDTW_CUDA(h, cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)smem));
+    CDTW_TRY(allow_smem(h, (const void*)k, smem));
     int per_sm = 0;
     CDTW_CUDA(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)k, 32 * wpb,
                                                                smem));

@@ -572,10 +572,7 @@ static int launch_stats(cdtw_handle h, const XT* x, int64_t N, int M, double* mu
         return CDTW_OK;
     }
     const size_t smem = tile_smem<XT, ST>(M);
-    if (smem > 48 * 1024)
-        CDTW_CUDA(h, cudaFuncSetAttribute((const void*)avg_std_kernel<XT, ST, INV>,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)smem));
+    CDTW_TRY(allow_smem(h, (const void*)avg_std_kernel<XT, ST, INV>, smem));
     avg_std_kernel<XT, ST, INV>
         <<<(unsigned)div_up(Nw, kTileWindows), kTileThreads, smem, h->stream>>>(x, N, M, mu, sigma);
     CDTW_LAUNCH(h, "avg_std_kernel");
@@ -598,10 +595,7 @@ int launch_rstd64(cdtw_handle h, const double* x, int64_t N, int M, double* rs) 
 int launch_prepare_queries(cdtw_handle h, const float* raw, const int64_t* offs,
                            const QueryPack* packs, int nq, int max_m) {
     const size_t smem = (size_t)max_m * (sizeof(double) + sizeof(float));
-    if (smem > 48 * 1024)
-        CDTW_CUDA(h, cudaFuncSetAttribute((const void*)prepare_queries_kernel,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)smem));
+    CDTW_TRY(allow_smem(h, (const void*)prepare_queries_kernel, smem));
     prepare_queries_kernel<<<nq, 256, smem, h->stream>>>(raw, offs, packs);
     CDTW_LAUNCH(h, "prepare_queries_kernel");
     return CDTW_OK;
@@ -609,10 +603,7 @@ int launch_prepare_queries(cdtw_handle h, const float* raw, const int64_t* offs,
 
 int launch_prepare_query(cdtw_handle h, const float* d_query_raw, int M, int W) {
     const size_t smem = (size_t)M * (sizeof(double) + sizeof(float));
-    if (smem > 48 * 1024)
-        CDTW_CUDA(h, cudaFuncSetAttribute((const void*)prepare_query_kernel,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)smem));
+    CDTW_TRY(allow_smem(h, (const void*)prepare_query_kernel, smem));
     prepare_query_kernel<<<1, 256, smem, h->stream>>>(d_query_raw, M, W, h->q);
     CDTW_LAUNCH(h, "prepare_query_kernel");
     return CDTW_OK;
