@@ -25,7 +25,8 @@ from typing import Callable, Iterable
 
 import numpy as np
 
-MAX_REGISTER_BAND = 96
+MAX_REGISTER_BAND = 106        # of the plain kernels (kMaxRegW, csrc/cdtw_reg.cuh)
+MAX_BATCH_REGISTER_BAND = 96   # of the batched tile kernels (kMaxBatchRegW, csrc/batch_reg.cuh)
 STRIP_ROWS = (1, 2, 4, 8, 16)
 TILE_CHOICES = (512, 1024, 2048)
 DEFAULT_ROWS_TILES = None  # the library's built-in rule when a bucket is untuned
@@ -50,7 +51,7 @@ def bucket(M: int, W: int) -> str:
 
 def batched_candidates(W: int) -> list[tuple[int, int]]:
     """(rows, tiles) pairs the batched search accepts for band W."""
-    rows = ([0] if W <= MAX_REGISTER_BAND else []) + [r for r in STRIP_ROWS if W >= r - 1]
+    rows = ([0] if W <= MAX_BATCH_REGISTER_BAND else []) + [r for r in STRIP_ROWS if W >= r - 1]
     return [(r, t) for r in rows for t in TILE_CHOICES]
 
 
@@ -66,6 +67,13 @@ def variant_candidates(W: int) -> list[str]:
     if lane_shape(W) is not None:
         out.append("lane")
     return out
+
+
+def builtin_variant(W: int) -> str:
+    """The library's own choice for band W (choose_variant in csrc/cdtw_reg.cu)."""
+    if W <= MAX_REGISTER_BAND:
+        return "register"
+    return "lane" if lane_shape(W) is not None else "strip16"
 
 
 def lane_shape(W: int):
@@ -121,7 +129,7 @@ def shapes_for(queries: list, bands: Iterable[int], table: dict):
             rows[i], tiles[i] = e["rows"], e["tiles"]
             hit = True
         else:  # the built-in rule for this query
-            rows[i] = 0 if w <= MAX_REGISTER_BAND else 16
+            rows[i] = 0 if w <= MAX_BATCH_REGISTER_BAND else 16
             tiles[i] = 1024
     return (rows, tiles) if hit else (None, None)
 
@@ -137,9 +145,12 @@ def tune_variants(bands: Iterable[int], measure: Callable[[int, str], float]) ->
 
 
 def apply_variants(handle, variants: dict) -> None:
-    """Set the tuned variant of every band on a Handle."""
+    """Set the tuned variant of every band on a Handle.  Where it is the
+    library's own choice the band stays on "auto", which also goes by the number
+    of windows."""
     for w, v in variants.items():
-        handle.set_band_variant(int(w), int(w), v)
+        w = int(w)
+        handle.set_band_variant(w, w, "auto" if v == builtin_variant(w) else v)
 
 
 # -- persistence ----------------------------------------------------------------
