@@ -162,6 +162,11 @@ bool lane_shape(int W, int* G, int* B) {
 
 int lane_qpad_min(int M, int W) { return M + 2 * W + 52; }
 
+int lane_block_windows(int W) {
+    int G, B;
+    return lane_shape(W, &G, &B) ? 2 * (kLaneThreads / G) : 0;
+}
+
 int launch_cdtw_lane(cdtw_handle h, const float* x, int64_t N, const double* mu,
                      const float* sigma, const int32_t* idx, int64_t L, bool euclid,
                      float* out) {

@@ -59,20 +59,39 @@ int choose_variant(cdtw_handle h, int W) {
     return v;
 }
 
-// The search's kernel: bands above kLaneSearchW over few windows keep the lane
-// groups, whose windows take a quarter of a thread's time each (M = 1000,
-// W = 100: 32k windows 1.06 ms on the register band and 1.00 on lane groups,
-// 262k 2.8 and 4.1).
-int search_variant(cdtw_handle h, int W, int64_t Nw) {
-    constexpr int kLaneSearchW = 96;
-    constexpr int64_t kLaneSearchWindows = 1 << 16;
-    const int v = choose_variant(h, W);
+// Bands that both the register band and the lane groups take, whose windows
+// take the lanes less time each: few of them are faster there.
+static bool few_on_lanes(cdtw_handle h, int W, int64_t windows, int64_t few) {
+    constexpr int kLaneMinW = 96;
     int G, B;
-    if (v == CDTW_VARIANT_REGISTER && W > kLaneSearchW && Nw < kLaneSearchWindows &&
-        h->band_variant[W] == CDTW_VARIANT_AUTO && lane_shape(W, &G, &B) &&
-        h->q.lq >= lane_qpad_min(h->q.M, W))
-        return CDTW_VARIANT_LANE;
-    return v;
+    return W > kLaneMinW && windows <= few && h->band_variant[W] == CDTW_VARIANT_AUTO &&
+           lane_shape(W, &G, &B) && h->q.lq >= lane_qpad_min(h->q.M, W);
+}
+
+// The search's kernel (M = 1000, W = 100: 32k windows 1.06 ms on the register
+// band and 1.00 on lane groups, 262k 2.8 and 4.1).
+int search_variant(cdtw_handle h, int W, int64_t Nw) {
+    const int v = choose_variant(h, W);
+    return v == CDTW_VARIANT_REGISTER && few_on_lanes(h, W, Nw, (1 << 16) - 1) ? CDTW_VARIANT_LANE
+                                                                              : v;
+}
+
+// The kernel of L listed windows, or of all L of them: the lane groups as long
+// as they need no more than a block an SM, two for the widest bands.  M = 1024,
+// us on the register band / lane groups, all windows (148 SMs: a block each up
+// to 9472 windows):
+//   windows  9000         10000        18000        19500         41000
+//   W = 97   495 / 401    494 / 608    505 / 606    790 / 941     1551 / 1492
+//   W = 102  591 / 435    592 / 638    619 / 640    841 / 1001    1656 / 1577
+//   W = 106  713 / 466    716 / 713    767 / 714    900 / 1102    1779 / 1746
+// (at 41000 the register band starts its second wave; M = 300 has it faster
+// there, 395 / 531.)
+static int windows_variant(cdtw_handle h, int W, int64_t L) {
+    constexpr int kTwoBlocksW = 105;
+    const int v = choose_variant(h, W);
+    const int64_t few =
+        (int64_t)h->sm_count * lane_block_windows(W) * (W >= kTwoBlocksW ? 2 : 1);
+    return v == CDTW_VARIANT_REGISTER && few_on_lanes(h, W, L, few) ? CDTW_VARIANT_LANE : v;
 }
 
 int launch_cdtw_strip_search(cdtw_handle h, const float* x, int64_t N, const double* mu,
@@ -115,7 +134,7 @@ int launch_cdtw_windows(cdtw_handle h, const float* x, int64_t N, const double* 
                         float* out) {
     const QueryPack& q = h->q;
     const int Nw = (int)(N - q.M + 1);
-    const int variant = q.qrev ? choose_variant(h, q.W) : CDTW_VARIANT_REGISTER;
+    const int variant = q.qrev ? windows_variant(h, q.W, L) : CDTW_VARIANT_REGISTER;
     if (variant == CDTW_VARIANT_LANE)
         return launch_cdtw_lane(h, x, N, mu, sigma, idx, L, euclid, out);
     if (variant != CDTW_VARIANT_REGISTER || q.W > kMaxRegW) {

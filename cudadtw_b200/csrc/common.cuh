@@ -449,6 +449,7 @@ int strip_rows_default(int W);
 // Lane-block kernels (cdtw_lane.cu): band spread over G lanes of B cells.
 bool lane_shape(int W, int* G, int* B);
 int lane_qpad_min(int M, int W);  // floats per query copy they read
+int lane_block_windows(int W);    // windows of one of their blocks; 0 outside their bands
 int launch_cdtw_lane(cdtw_handle h, const float* x, int64_t N, const double* mu,
                      const float* sigma, const int32_t* idx, int64_t L, bool euclid, float* out);
 int launch_cdtw_lane_search(cdtw_handle h, const float* x, int64_t N, const double* mu,
