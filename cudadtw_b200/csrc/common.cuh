@@ -128,9 +128,9 @@ int run_topk_device(cdtw_handle h, const float* x, int64_t N, const double* mu,
 // topk_device.cu
 int launch_topk_threshold(cdtw_handle h, const float* sd, int nseg, const float* prev_d,
                           const int* prev_n, int k2, unsigned long long* key, float* t_out);
-int launch_topk_greedy(cdtw_handle h, const unsigned long long* hits, const int* nh, int cap,
-                       int k2, int M, int* acc, int32_t* picks, float* pick_d, int* npicks,
-                       int* status);
+int launch_topk_greedy(cdtw_handle h, unsigned long long* hits, unsigned long long* spare,
+                       const int* nh, int cap, int k2, int M, int* acc, int32_t* picks,
+                       float* pick_d, int* npicks, int* status);  // spare: room for the hits
 // pairwise cDTW forward / backward (pair.cu)
 void pair_shape(int L, int W, int* G, int* C);
 size_t pair_dirs_words(int L, int W);

@@ -857,8 +857,10 @@ int run_topk_device(cdtw_handle h, const float* x, int64_t N, const double* mu,
     CDTW_CUDA(h, cudaMemsetAsync(dw.acc, 0xff, sizeof(int) * ((size_t)dw.nbuckets + 2),
                                  h->stream));
     if (ctr_out) *ctr_out = ws.ctr;
-    return launch_topk_greedy(h, tw.hits, tw.nh, (int)cap, k2, M, dw.acc, picks, pick_d, npicks,
-                              status);
+    // (the candidates are done with: their list is the greedy's second one)
+    static_assert(sizeof(Cand) >= sizeof(unsigned long long), "room for a key per candidate");
+    return launch_topk_greedy(h, tw.hits, (unsigned long long*)ws.q2, tw.nh, (int)cap, k2, M,
+                              dw.acc, picks, pick_d, npicks, status);
 }
 
 size_t search_workspace_bytes(int64_t N, int M, int W) {

@@ -12,7 +12,9 @@
 // greedy consumes them: one block repeatedly radix-selects the next B
 // smallest keys, sorts them in shared memory, tests them against the
 // accepted windows in parallel and resolves the few that remain in key order
-// with one warp (ballots over 32 keys at a time).
+// with one warp (ballots over 32 keys at a time).  Where many more picks are
+// wanted than a round makes, the keys that are consumed or overlap a pick are
+// dropped after each round, so that the next ones read a shorter list.
 #include "common.cuh"
 
 namespace cdtw {
@@ -117,9 +119,10 @@ __device__ __forceinline__ bool overlaps_accepted(const int* acc, int w, int M) 
 }
 
 __global__ void __launch_bounds__(kSelThreads)
-topk_greedy_kernel(const unsigned long long* __restrict__ hits, const int* __restrict__ nh_ptr,
-                   int cap, int k2, int M, int* __restrict__ acc, int32_t* __restrict__ picks,
-                   float* __restrict__ pick_d, int* __restrict__ npicks, int* __restrict__ status) {
+topk_greedy_kernel(unsigned long long* hits, unsigned long long* spare,
+                   const int* __restrict__ nh_ptr, int cap, int k2, int M, int* __restrict__ acc,
+                   int32_t* __restrict__ picks, float* __restrict__ pick_d,
+                   int* __restrict__ npicks, int* __restrict__ status) {
     __shared__ unsigned long long keys[kGreedyB];
     __shared__ int hist[256];
     __shared__ int ulist[kSelThreads];
@@ -135,7 +138,7 @@ topk_greedy_kernel(const unsigned long long* __restrict__ hits, const int* __res
         }
         return;
     }
-    const int nh = nh_all;
+    int nh = nh_all;
     if (tid == 0) {
         s_np = 0;
         *status = 0;
@@ -146,6 +149,7 @@ topk_greedy_kernel(const unsigned long long* __restrict__ hits, const int* __res
     // the windows around a match are hits too: about 16 keys a pick first
     int chunk = min(3 * kGreedyB / 4, max(512, 16 * min(k2, kGreedyB)));
     while (consumed < nh && s_np < k2) {
+        const int np0 = s_np;
         const int take = min(chunk, nh - consumed);
         chunk = 3 * kGreedyB / 4;
         // hi: a bound with at least `take` and at most kGreedyB keys in [lo, hi]
@@ -266,6 +270,29 @@ topk_greedy_kernel(const unsigned long long* __restrict__ hits, const int* __res
         }
         consumed += cnt;
         lo = hi + 1;
+        // Several more rounds to come: the keys still open go to the other
+        // list.  (Without it k = 32768 over 2^21 hits of M = 64 takes 680
+        // rounds over all of them.)
+        if (nh - consumed > kGreedyB && k2 - s_np > 2 * (s_np - np0)) {
+            if (tid == 0) s_cnt = 0;
+            __syncthreads();
+            for (int i0 = 32 * warp; i0 < nh; i0 += kSelThreads) {
+                const unsigned long long k = i0 + lane < nh ? hits[i0 + lane] : 0ull;
+                const bool keep =
+                    i0 + lane < nh && k >= lo && !overlaps_accepted(acc, (int)(uint32_t)k, M);
+                const unsigned bal = __ballot_sync(0xffffffffu, keep);
+                int at = 0;
+                if (lane == 0) at = atomicAdd(&s_cnt, __popc(bal));
+                at = __shfl_sync(0xffffffffu, at, 0);
+                if (keep) spare[at + __popc(bal & ((1u << lane) - 1))] = k;
+            }
+            __syncthreads();
+            nh = s_cnt;
+            consumed = 0;
+            unsigned long long* const other = hits;
+            hits = spare;
+            spare = other;
+        }
         __syncthreads();
     }
     if (tid == 0) *npicks = s_np;
@@ -281,11 +308,11 @@ int launch_topk_threshold(cdtw_handle h, const float* sd, int nseg, const float*
     return CDTW_OK;
 }
 
-int launch_topk_greedy(cdtw_handle h, const unsigned long long* hits, const int* nh, int cap,
-                       int k2, int M, int* acc, int32_t* picks, float* pick_d, int* npicks,
-                       int* status) {
-    topk_greedy_kernel<<<1, kSelThreads, 0, h->stream>>>(hits, nh, cap, k2, M, acc, picks, pick_d,
-                                                        npicks, status);
+int launch_topk_greedy(cdtw_handle h, unsigned long long* hits, unsigned long long* spare,
+                       const int* nh, int cap, int k2, int M, int* acc, int32_t* picks,
+                       float* pick_d, int* npicks, int* status) {
+    topk_greedy_kernel<<<1, kSelThreads, 0, h->stream>>>(hits, spare, nh, cap, k2, M, acc, picks,
+                                                        pick_d, npicks, status);
     CDTW_LAUNCH(h, "topk_greedy_kernel");
     return CDTW_OK;
 }
