@@ -365,7 +365,7 @@ class Handle:
         return int(self._lib.cdtw_pair_workspace_bytes(n, L, W, flags, int(with_path)))
 
     def pair_last_mode(self) -> str:
-        """"recompute" or "store": how the last pair_fwd with a path recorded it."""
+        """"recompute" or "store": whose scratch the last pair_fwd with a path took."""
         r = ctypes.c_int()
         self._check(self._lib.cdtw_pair_last_mode(self._h, ctypes.byref(r)))
         return "recompute" if r.value else "store"

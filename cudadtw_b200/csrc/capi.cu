@@ -773,7 +773,7 @@ int cdtw_pair_fwd(cdtw_handle h, const float* d_q, const float* d_s, int64_t n, 
     CDTW_TRY(ensure_workspace(
         h, pair_carve(n, L, W, flags, d_path != nullptr, recompute, &o_zq, &o_zs, &o_dirs)));
     const bool store = flags & CDTW_PAIR_STORE_DIRS;
-    h->last_pair_recompute = recompute ? 1 : 0;  // or set by launch_pair_fwd
+    h->last_pair_recompute = recompute ? 1 : 0;
     char* ws = (char*)h->ws;
     double* hdr = (double*)d_path;
     uint32_t* rows = d_path ? (uint32_t*)((char*)d_path + (size_t)n * 32) : nullptr;

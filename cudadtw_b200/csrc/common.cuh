@@ -86,7 +86,7 @@ struct cdtw_handle_s {
     int64_t last_counts[4] = {0, 0, 0, 0};
     // the last search's best distance lies below the largest LB_Kim
     int last_flag = 0;
-    // the last cdtw_pair_fwd with a path record recomputed from checkpoints
+    // the last cdtw_pair_fwd ran in the recomputation's smaller scratch
     int last_pair_recompute = 0;
     // cDTW kernel variant per band (0 = built-in rule); set by the autotuner
     unsigned char band_variant[CDTW_MAX_QUERY] = {0};
@@ -144,7 +144,7 @@ int launch_pair_znorm(cdtw_handle h, const float* q, const float* s, int64_t n, 
 // path record) lane groups of 32 with the fewest cells per lane -- the
 // shortest step, for a handful of pairs.  store: a path record keeps direction
 // bits in dirs; otherwise dirs holds checkpoints where that is the faster way
-// (pair_auto_mode; h->last_pair_recompute is set then).
+// (pair_auto_mode).
 int launch_pair_fwd(cdtw_handle h, const float* zq, const float* zs, int64_t n, int L, int W,
                     bool euclid, float* D, uint32_t* dirs, uint32_t* rows, uint32_t* cols,
                     int64_t qstride = -1, const int* gate = nullptr, int gate_max = 0,

@@ -341,7 +341,6 @@ int launch_pair_fwd(cdtw_handle h, const float* zq, const float* zs, int64_t n, 
     pair_shape(L, W, &G, &C);
     if (C > 16) return set_error(h, CDTW_EUNSUPPORTED, "pair band W=%d exceeds 511", W);
     const int mode = rows && cols && dirs && !store ? pair_auto_mode(h, n, L, W) : 0;
-    if (mode) h->last_pair_recompute = 1;
     if (mode == 2)
         return launch_pair_fwd_ckpt(h, zq, zs, n, L, W, euclid, D, (float*)dirs, rows, cols);
     if (!rows && wide) {

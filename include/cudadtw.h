@@ -365,8 +365,9 @@ size_t cdtw_pair_workspace_bytes(int64_t n, int L, int W, int flags, int with_pa
  * the path's surroundings are recomputed.  No reference counterpart (the DP of
  * include/cdtw.cuh:24-88 returns distances only). */
 
-/* 1 when the last cdtw_pair_fwd with a path record on this handle recomputed
- * from checkpoints, 0 when it stored direction bits.  No reference
+/* 1 when the last cdtw_pair_fwd with a path record on this handle ran in the
+ * recomputation's smaller scratch (forced, or by the memory limit), 0 when in
+ * that of stored directions, whichever of the two that held.  No reference
  * counterpart. */
 int cdtw_pair_last_mode(cdtw_handle h, int* recompute);
 
