@@ -247,9 +247,13 @@ void pair_shape(int L, int W, int* G, int* C) {
 
 // Shared-record mode of the forward with a path: the record stays in shared
 // memory when it takes at most 512 bytes per lane (C <= 4, one byte per lane
-// and anti-diagonal) and the block's records and move logs leave room for 3
-// blocks per SM.  recb / logb: bytes per group, with strides of 32 (mod 128)
-// bytes so the groups of a warp sit on different shared-memory banks.
+// and anti-diagonal) and the block's records and move logs, without the pads
+// that launch_pair_fwd puts in front of the records, leave room for 3 blocks per
+// SM; with them some sizes have 2.  (Pads inside the strides instead: 32768
+// pairs of 220, W = 11, 399 -> 347 us, but of 150, W = 7, 259 -> 332 and of 78,
+// W = 3, 65536 pairs, 316 -> 382.)  recb / logb: bytes per group, with strides of
+// 32 (mod 128) bytes so the groups of a warp sit on different shared-memory
+// banks.
 static bool pair_shared_record(int L, int G, int C, int* recb, int* logb, size_t* bytes) {
     const int K = 2 * L - 1;
     *recb = (int)round_up((int64_t)K * G, 128) + 32;
