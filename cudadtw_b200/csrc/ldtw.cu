@@ -112,10 +112,12 @@ __device__ __forceinline__ float lcost_ref(float d) {
 // System/6000 processor", IBM J. R&D 34 (1990).  RN(a y) is within 1.5 ulp, so
 // one such step brings it within one and the second gives the quotient (zero
 // stays zero).  That holds while nothing under- or overflows, which `exact`
-// grants for every sample of the window: sd in [2^-60, 2^60] and |avg| in
-// [2^-70, 2^100], so a nonzero a = x - avg is at least 2^-95, a residual a
-// multiple of 2^-141 and |q| below 2^25 (sd is at least 2^-13 max|x| / sqrt(M)
-// where it is not 1).  Windows outside divide.
+// grants for every sample of the window: sd in [2^-60, 2^40] and |avg| in
+// [2^-60, 2^100], so a nonzero a = x - avg is at least 2^-84, q at least 2^-125
+// and a residual a multiple of 2^-132.  The variance is the rounded difference
+// of a 24-bit mean of squares and a 48-bit square, so where it is positive it is
+// at least 2^-48 of that mean, sd at least 2^-25 max|x| / sqrt(M) and |q| below
+// 2^33 (sd = 1 otherwise: |q| below 2^108).  Windows outside divide.
 struct RefNorm {
     float avg, sd, y;
     bool exact;
@@ -126,7 +128,7 @@ __device__ __forceinline__ RefNorm make_ref_norm(float avg, float sd) {
     n.sd = sd;
     n.y = __frcp_rn(sd);
     const float m = fabsf(avg);
-    n.exact = sd >= 0x1p-60f && sd <= 0x1p60f && m >= 0x1p-70f && m <= 0x1p100f;
+    n.exact = sd >= 0x1p-60f && sd <= 0x1p40f && m >= 0x1p-60f && m <= 0x1p100f;
     return n;
 }
 template <bool EXACT>
