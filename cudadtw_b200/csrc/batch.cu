@@ -237,7 +237,7 @@ batch_strip_kernel(const BatchArgs b) {
 }  // namespace
 
 size_t batch_smem_bytes(int tmax, int mmax, int lq4max) {
-    return (size_t)tmax * (8 + 4 * 6) + (size_t)(tmax + mmax) * 4 + 16 + (size_t)lq4max * 64 +
+    return (size_t)tmax * (8 + 4 * 6) + (size_t)(tmax + mmax) * 4 + 16 + (size_t)lq4max * 16 +
            (size_t)mmax * 8 + 64;
 }
 

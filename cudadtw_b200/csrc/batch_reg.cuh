@@ -17,8 +17,8 @@ __global__ void __launch_bounds__(kBatchThreads)
 batch_reg_kernel(const BatchArgs b) {
     extern __shared__ __align__(16) unsigned char smem[];
     const TileSmem ts = carve_tile(smem, b.tmax, b.mmax);
-    float4* sq4 = ts.tail;                             // lq4max (of 4 * lq4max)
-    float2* senv = (float2*)(sq4 + 4 * b.lq4max);      // reg_env_len(mmax)
+    float4* sq4 = ts.tail;                         // lq4max
+    float2* senv = (float2*)(sq4 + b.lq4max);      // reg_env_len(mmax)
     __shared__ int s_item, s_na, s_nb, s_next;
     const int tid = threadIdx.x, lane = tid & 31;
     int q, tile;

@@ -41,43 +41,16 @@ template <bool EU>
 __global__ void __launch_bounds__(256)
 lb_kim_kernel(const float* __restrict__ x, const double* __restrict__ mu,
               const float* __restrict__ sigma, const float* __restrict__ zq, int M, int Nw,
-              const int32_t* __restrict__ idx, int L, float* __restrict__ out,
-              unsigned long long* __restrict__ seeds, unsigned* __restrict__ bmax) {
-    __shared__ unsigned long long best;
-    __shared__ unsigned vmax;
-    if (seeds && threadIdx.x == 0) {
-        best = ~0ull;
-        vmax = 0u;
-    }
-    if (seeds) __syncthreads();
+              const int32_t* __restrict__ idx, int L, float* __restrict__ out) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    float v = CDTW_INF;
-    int w = -1;
-    if (t < L) {
-        w = idx ? idx[t] : t;
-        if (w >= 0 && w < Nw) {
-            const Norm nm = make_norm(mu[w], sigma[w]);
-            v = lb_kim_window<EU>(x + w, nm, zq, M);
-        } else {
-            v = __int_as_float(0x7fc00000);
-        }
-        out[t] = v;
+    if (t >= L) return;
+    const int w = idx ? idx[t] : t;
+    float v = __int_as_float(0x7fc00000);
+    if (w >= 0 && w < Nw) {
+        const Norm nm = make_norm(mu[w], sigma[w]);
+        v = lb_kim_window<EU>(x + w, nm, zq, M);
     }
-    if (seeds) {  // the block's smallest bound: a seed window for the search
-        const bool ok = t < L && w >= 0 && w < Nw && v == v;
-        const unsigned long long k = warp_min_key(ok, v, (uint32_t)w);
-        // and its largest (bounds are >= 0: their bits order as unsigned)
-        const unsigned mx = __reduce_max_sync(0xffffffffu, ok ? __float_as_uint(v) : 0u);
-        if ((threadIdx.x & 31) == 0) {  // one shared atomic of each kind per warp
-            if (k != ~0ull) atomicMin(&best, k);
-            atomicMax(&vmax, mx);
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            seeds[blockIdx.x] = best;
-            bmax[blockIdx.x] = vmax;
-        }
-    }
+    out[t] = v;
 }
 
 // Stream envelope of the reverse LB_Keogh (the data envelope of
@@ -354,8 +327,7 @@ int launch_lb_kim_all(cdtw_handle h, const float* x, int64_t N, const double* mu
 }
 
 int launch_lb_kim(cdtw_handle h, const float* x, int64_t N, const double* mu, const float* sigma,
-                  const int32_t* idx, int64_t L, bool euclid, float* out,
-                  unsigned long long* seeds, unsigned* bmax) {
+                  const int32_t* idx, int64_t L, bool euclid, float* out) {
     const QueryPack& q = h->q;
     if (q.M < 11)
         return set_error(h, CDTW_EINVAL,
@@ -365,10 +337,10 @@ int launch_lb_kim(cdtw_handle h, const float* x, int64_t N, const double* mu, co
     const unsigned blocks = (unsigned)div_up(L, 256);
     if (euclid)
         lb_kim_kernel<true><<<blocks, 256, 0, h->stream>>>(x, mu, sigma, q.zq, q.M, Nw, idx,
-                                                            (int)L, out, seeds, bmax);
+                                                            (int)L, out);
     else
         lb_kim_kernel<false><<<blocks, 256, 0, h->stream>>>(x, mu, sigma, q.zq, q.M, Nw, idx,
-                                                             (int)L, out, seeds, bmax);
+                                                             (int)L, out);
     CDTW_LAUNCH(h, "lb_kim_kernel");
     return CDTW_OK;
 }

@@ -467,8 +467,7 @@ int choose_variant(cdtw_handle h, int W);
 int search_variant(cdtw_handle h, int W, int64_t Nw);
 int max_batch_register_band();  // of the batched tile kernels
 int launch_lb_kim(cdtw_handle h, const float* x, int64_t N, const double* mu, const float* sigma,
-                  const int32_t* idx, int64_t L, bool euclid, float* out,
-                  unsigned long long* seeds = nullptr, unsigned* bmax = nullptr);
+                  const int32_t* idx, int64_t L, bool euclid, float* out);
 // The search's first pass: LB_Kim of every window into out (256-byte
 // aligned), per 256 windows the smallest (seeds) and the largest (bmax).
 int launch_lb_kim_all(cdtw_handle h, const float* x, int64_t N, const double* mu,
