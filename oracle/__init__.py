@@ -13,6 +13,7 @@ import os
 import re
 import subprocess
 import tempfile
+import unittest
 
 import numpy as np
 
@@ -208,11 +209,21 @@ _DIST = re.compile(r"Distance\s*:\s*([-+0-9.eEinfa]+)")
 _TIME = re.compile(r"Total Execution Time\s*:\s*([0-9.eE+-]+)")
 
 
-def _run_ucr(binary: str, args: list[str]):
-    path = os.path.join(REF_DIR, binary)
+class ReferenceMissing(unittest.SkipTest, FileNotFoundError):
+    """A program built from the reference's sources is not there; a test that
+    needs it is skipped (pytest takes unittest's SkipTest as its own)."""
+
+
+def _ref_program(name: str) -> str:
+    path = os.path.join(REF_DIR, name)
     if not os.path.exists(path):
-        raise FileNotFoundError(f"{path} missing: run `make -C oracle ref` where the "
-                                "reference sources are available")
+        raise ReferenceMissing(f"{path} missing: run `make -C oracle ref` where the "
+                               "reference sources are available")
+    return path
+
+
+def _run_ucr(binary: str, args: list[str]):
+    path = _ref_program(binary)
     out = subprocess.run([path] + args, check=True, stdout=subprocess.PIPE,
                          stderr=subprocess.DEVNULL, text=True).stdout
     loc = int(_LOC.search(out).group(1))
@@ -252,13 +263,12 @@ class UcrShards:
 
     def __init__(self, x: np.ndarray, shards: int | None = None, max_m: int = 8192):
         self.x = x
-        self.path = os.path.join(REF_DIR, "UCR_DTW_BIN")
-        if not os.path.exists(self.path):
-            raise FileNotFoundError(f"{self.path} missing: run `make -C oracle ref`")
         self.shards = max(1, min(shards or (os.cpu_count() or 1), x.size))
         self.bounds = [x.size * s // self.shards for s in range(self.shards + 1)]
         self.dir = tempfile.TemporaryDirectory()
         self.files = []
+        if not os.path.exists(os.path.join(REF_DIR, "UCR_DTW_BIN")):
+            return  # search() says so; what needs the stream alone goes on
         for s in range(self.shards):
             a = self.bounds[s]
             fp = os.path.join(self.dir.name, f"data{s}.f64")
@@ -275,6 +285,7 @@ class UcrShards:
         """Returns (location, distance as UCR printed it, wall seconds,
         [per-shard clock() seconds])."""
         import time
+        path = _ref_program("UCR_DTW_BIN")
         m = q.size
         nw = self.x.size - m + 1
         qp = os.path.join(self.dir.name, "query.f64")
@@ -285,7 +296,7 @@ class UcrShards:
             if b > a:
                 jobs.append((a, self.files[s], b - a + m - 1))
         t0 = time.perf_counter()
-        procs = [subprocess.Popen([self.path, fp, qp, str(m), ucr_band_arg(w, m), str(n)],
+        procs = [subprocess.Popen([path, fp, qp, str(m), ucr_band_arg(w, m), str(n)],
                                   stdout=subprocess.PIPE, stderr=subprocess.DEVNULL, text=True)
                  for _, fp, n in jobs]
         outs = [p.communicate()[0] for p in procs]
@@ -320,9 +331,7 @@ def ref_ldtw(q: np.ndarray, x: np.ndarray, w: int, znorm: bool = True):
     include/ldtw.cuh, built into _ref/ref_ldtw) on every window, with the
     inputs its GPU-ldtw.cu makes (FP32 query z-normalisation, avg_std window
     statistics).  Returns (float32 costs per window, determine_min's index)."""
-    path = os.path.join(REF_DIR, "ref_ldtw")
-    if not os.path.exists(path):
-        raise FileNotFoundError(f"{path} missing: run `make -C oracle ref`")
+    path = _ref_program("ref_ldtw")
     with tempfile.TemporaryDirectory() as d:
         qp, xp, rp = (os.path.join(d, n) for n in ("q.bin", "s.bin", "r.bin"))
         np.ascontiguousarray(q, np.float32).tofile(qp)
