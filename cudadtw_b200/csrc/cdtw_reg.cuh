@@ -328,9 +328,13 @@ __device__ __forceinline__ float reg_window_dtw(const float4* sq4, const float2*
 // list, skip those whose lower bound already exceeds the best-so-far, run the
 // register-band DTW with early abandoning, and fold results into *key by a
 // packed (distance, window) atomicMin, so ties keep the lowest window (or
-// append them to a hit list, report_window).
+// append them to a hit list, report_window).  One block an SM in the launch
+// bounds: left to itself the compiler holds the registers down for more warps
+// and the rows' chains no longer overlap (W = 60, 168 registers instead of 180:
+// 4 candidates of M = 300 151 us and 95, 100000 351 and 249; W = 25 78 and 50,
+// 160 and 159).
 template <int W, bool EU>
-__global__ void __launch_bounds__(kRegBlock)
+__global__ void __launch_bounds__(kRegBlock, 1)
 cdtw_reg_search_kernel(const float* __restrict__ x, const double* __restrict__ mu,
                        const float* __restrict__ sigma, const float4* __restrict__ qpad4, int lq4,
                        const float2* __restrict__ qenv, int M, const Cand* __restrict__ cands,
