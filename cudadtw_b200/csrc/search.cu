@@ -218,9 +218,10 @@ __device__ __forceinline__ float warp_sum_f(float v) {
 // schedulers busy: searches with 29k LB_Kim survivors, M = 1000, W = 50, 523 ->
 // 456 us; with 125k, M = 128, 134 -> 173), above that a thread.
 constexpr int kFilterWarps = 1 << 15;
+constexpr int kFilterThreads = 256;
 
 template <bool EU>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(kFilterThreads)
 keogh_filter_kernel(const float* __restrict__ x, const double* __restrict__ mu,
                     const float* __restrict__ sigma, const float* __restrict__ zq,
                     const float2* __restrict__ qenv, const float2* __restrict__ xenv,
@@ -234,13 +235,19 @@ keogh_filter_kernel(const float* __restrict__ x, const double* __restrict__ mu,
     const int lane = threadIdx.x & 31;
     if (n1 <= kFilterWarps) {
         // a warp per window, lanes over its samples; both bounds abandoned
-        // every 128.  A warp takes neighbouring entries and appends their
-        // survivors together (lane c keeps the c-th): the search kernels' warps
-        // want neighbouring windows.
-        const int nwarps = (int)(gridDim.x * blockDim.x) >> 5;
+        // every 128.  A block takes neighbouring entries, a warp `per` of them
+        // (lane c keeps its c-th survivor), and appends the survivors in their
+        // order: the search kernels' warps want neighbouring windows, which are
+        // abandoned together (19k survivors, M = 700, W = 140, lane groups: 646
+        // us in groups of 32, 755 with each warp's three by themselves, 590
+        // so).
+        __shared__ int s_kept[kFilterThreads / 32], s_at;
+        constexpr int wpb = kFilterThreads / 32;
+        const int wid = threadIdx.x >> 5;
+        const int nwarps = (int)gridDim.x * wpb;
         const int per = min(32, (n1 + nwarps - 1) / nwarps);
-        const int first = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * per;
-        for (int i0 = first; i0 < n1; i0 += nwarps * per) {
+        for (int b0 = (int)blockIdx.x * wpb * per; b0 < n1; b0 += nwarps * per) {
+            const int i0 = b0 + wid * per;
             int kept = 0;
             Cand mine;
             for (int i = i0; i < min(i0 + per, n1); ++i) {
@@ -284,12 +291,19 @@ keogh_filter_kernel(const float* __restrict__ x, const double* __restrict__ mu,
                     ++kept;
                 }
             }
-            if (kept) {
-                int at = 0;
-                if (lane == 0) at = atomicAdd(n2, kept);
-                at = __shfl_sync(0xffffffffu, at, 0);
-                if (lane < kept) q2[at + lane] = mine;
+            if (lane == 0) s_kept[wid] = kept;
+            __syncthreads();
+            int before = 0, all = 0;
+#pragma unroll
+            for (int w = 0; w < wpb; ++w) {
+                const int k = s_kept[w];
+                before += w < wid ? k : 0;
+                all += k;
             }
+            if (threadIdx.x == 0 && all) s_at = atomicAdd(n2, all);
+            __syncthreads();
+            if (lane < kept) q2[s_at + before + lane] = mine;
+            __syncthreads();  // both are written again by the next round
         }
         return;
     }
@@ -619,11 +633,11 @@ int launch_keogh(cdtw_handle h, const float* x, int64_t N, const double* mu, con
     CDTW_TRY(launch_stream_envelope(h, x, N, W, ws.envscratch, ws.xenv, ws.ctr + 0, sparse_max));
     const int grid = h->sm_count * 8;
     if (euclid)
-        keogh_filter_kernel<true><<<grid, 256, 0, h->stream>>>(
+        keogh_filter_kernel<true><<<grid, kFilterThreads, 0, h->stream>>>(
             x, mu, sigma, q.zq, q.env, ws.xenv, ws.lbkim, M, ws.q1, ws.ctr + 0, ws.key, ws.q2,
             ws.ctr + 1, sparse_max);
     else
-        keogh_filter_kernel<false><<<grid, 256, 0, h->stream>>>(
+        keogh_filter_kernel<false><<<grid, kFilterThreads, 0, h->stream>>>(
             x, mu, sigma, q.zq, q.env, ws.xenv, ws.lbkim, M, ws.q1, ws.ctr + 0, ws.key, ws.q2,
             ws.ctr + 1, sparse_max);
     CDTW_LAUNCH(h, "keogh_filter_kernel");
