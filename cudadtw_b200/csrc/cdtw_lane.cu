@@ -131,6 +131,7 @@ int fill_lane_args(cdtw_handle h, const float* x, int64_t N, const double* mu,
     a->count = nullptr;
     a->work = nullptr;
     a->nsm = h->sm_count;
+    a->gate = INT32_MAX;
     a->key = nullptr;
     return CDTW_OK;
 }
@@ -193,7 +194,7 @@ int launch_cdtw_lane(cdtw_handle h, const float* x, int64_t N, const double* mu,
 int launch_cdtw_lane_search(cdtw_handle h, const float* x, int64_t N, const double* mu,
                             const float* sigma, const Cand* cands, const int* count, int* work,
                             int max_count, bool euclid, unsigned long long* key,
-                            const HitSink& sink) {
+                            const HitSink& sink, int gate) {
     if (max_count <= 0) return CDTW_OK;
     LaneArgs a;
     CDTW_TRY(fill_lane_args(h, x, N, mu, sigma, &a));
@@ -203,6 +204,7 @@ int launch_cdtw_lane_search(cdtw_handle h, const float* x, int64_t N, const doub
     a.count = count;
     a.work = work;
     a.nsm = h->sm_count;
+    a.gate = gate;
     a.key = key;
     a.sink = sink;
     const LaneKernel k = euclid ? lane_kernels().seu[B] : lane_kernels().smh[B];

@@ -63,6 +63,7 @@ struct LaneArgs {
     const int* count;
     int* work;
     int nsm;  // SMs of the device
+    int gate;  // candidates above which the search kernel does nothing
     unsigned long long* key;
     HitSink sink;
 };
@@ -347,13 +348,14 @@ template <int B, bool EU>
 __global__ void __launch_bounds__(kLaneThreads)
 cdtw_lane_search_kernel(const LaneArgs a) {
     extern __shared__ float4 lsq4[];
+    const int n = *(const volatile int*)a.count;
+    if (n > a.gate) return;  // the register band takes them
     lane_stage_query(a, lsq4);
     const int G = a.G;
     const int lane = threadIdx.x & 31;
     const int g = lane & (G - 1);
     const int h = lane >> a.lgG;  // group in warp
     const int per_warp = 64 >> a.lgG;
-    const int n = *(const volatile int*)a.count;
     for (int base = first_batch(a.work, per_warp, a.nsm); base < n;
          base = next_batch(a.work, per_warp)) {
         const int i0 = base + 2 * h, i1 = base + 2 * h + 1;

@@ -68,12 +68,16 @@ static bool few_on_lanes(cdtw_handle h, int W, int64_t windows, int64_t few) {
            lane_shape(W, &G, &B) && h->q.lq >= lane_qpad_min(h->q.M, W);
 }
 
-// The search's kernel (M = 1000, W = 100: 32k windows 1.06 ms on the register
-// band and 1.00 on lane groups, 262k 2.8 and 4.1).
+// Candidates of a search up to which the lane groups are the faster (M = 1000,
+// W = 100: 9827 survivors of 300k windows 800 us on the register band and 460 on
+// lane groups, 32k windows 1060 and 1000, 262k 2800 and 4100).
+constexpr int kLaneCandidates = 1 << 15;
+
 int search_variant(cdtw_handle h, int W, int64_t Nw) {
     const int v = choose_variant(h, W);
-    return v == CDTW_VARIANT_REGISTER && few_on_lanes(h, W, Nw, (1 << 16) - 1) ? CDTW_VARIANT_LANE
-                                                                              : v;
+    return v == CDTW_VARIANT_REGISTER && few_on_lanes(h, W, Nw, kLaneCandidates)
+               ? CDTW_VARIANT_LANE
+               : v;
 }
 
 // The kernel of L listed windows, or of all L of them: the lane groups as long
@@ -113,6 +117,14 @@ int launch_cdtw_search(cdtw_handle h, const float* x, int64_t N, const double* m
         return launch_cdtw_strip_search(h, x, N, mu, sigma, cands, count, work, max_count,
                                         euclid, variant == CDTW_VARIANT_STRIP16 ? 16 : 32, key,
                                         sink);
+    // their number is known on the device only: both are launched, each returns
+    // at once where the other takes them
+    int gate = -1;
+    if (few_on_lanes(h, q.W, 0, 0)) {
+        gate = kLaneCandidates;
+        CDTW_TRY(launch_cdtw_lane_search(h, x, N, mu, sigma, cands, count, work,
+                                         std::min(max_count, gate), euclid, key, sink, gate));
+    }
     RegSearchKernel k = euclid ? reg_kernels().seu[q.W] : reg_kernels().smh[q.W];
     const int lq4 = q.lq / 4;
     const size_t smem = (size_t)q.lq * sizeof(float) + (size_t)reg_env_len(q.M) * sizeof(float2);
@@ -124,7 +136,8 @@ int launch_cdtw_search(cdtw_handle h, const float* x, int64_t N, const double* m
     const unsigned blocks = (unsigned)std::max<int64_t>(
         1, std::min<int64_t>(want, (int64_t)std::max(per_sm, 1) * h->sm_count));
     k<<<blocks, kRegBlock, smem, h->stream>>>(x, mu, sigma, (const float4*)q.qpad, lq4, q.env,
-                                              q.M, cands, count, work, key, sink, h->sm_count);
+                                              q.M, cands, count, work, key, sink, h->sm_count,
+                                              gate);
     CDTW_LAUNCH(h, "cdtw_reg_search_kernel");
     return CDTW_OK;
 }

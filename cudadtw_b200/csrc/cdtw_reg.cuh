@@ -339,14 +339,16 @@ cdtw_reg_search_kernel(const float* __restrict__ x, const double* __restrict__ m
                        const float* __restrict__ sigma, const float4* __restrict__ qpad4, int lq4,
                        const float2* __restrict__ qenv, int M, const Cand* __restrict__ cands,
                        const int* __restrict__ count, int* __restrict__ work,
-                       unsigned long long* __restrict__ key, const HitSink sink, int nsm) {
+                       unsigned long long* __restrict__ key, const HitSink sink, int nsm,
+                       int gate) {
     extern __shared__ float4 sq4[];
+    const int n = *(const volatile int*)count;
+    if (n <= gate) return;  // the lane groups take them
     float2* senv = (float2*)(sq4 + lq4);
     for (int e = threadIdx.x; e < lq4; e += blockDim.x) sq4[e] = qpad4[e];
     reg_stage_env(senv, qenv, M);
     __syncthreads();
     const int lane = threadIdx.x & 31;
-    const int n = *(const volatile int*)count;
     for (int base = first_batch(work, 32, nsm); base < n; base = next_batch(work, 32)) {
         const int i = base + lane;
         Cand c;
@@ -366,7 +368,7 @@ using RegKernel = void (*)(const float*, const double*, const float*, const floa
                            int, const int32_t*, int, float*);
 using RegSearchKernel = void (*)(const float*, const double*, const float*, const float4*, int,
                                  const float2*, int, const Cand*, const int*, int*,
-                                 unsigned long long*, const HitSink, int);
+                                 unsigned long long*, const HitSink, int, int);
 
 // Instantiates the one-window and the search kernels for bands LO..HI into the
 // dispatch tables.

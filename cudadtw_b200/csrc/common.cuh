@@ -455,7 +455,7 @@ int launch_cdtw_lane(cdtw_handle h, const float* x, int64_t N, const double* mu,
 int launch_cdtw_lane_search(cdtw_handle h, const float* x, int64_t N, const double* mu,
                             const float* sigma, const Cand* cands, const int* count, int* work,
                             int max_count, bool euclid, unsigned long long* key,
-                            const HitSink& sink);
+                            const HitSink& sink, int gate = INT32_MAX);
 // floats per shifted query copy (QueryPack::lq) of a handle's query pack
 inline int qpad_len(int M, int W) { return (int)(((int64_t)M + 2 * W + 56 + 3) / 4 * 4); }
 // Kernel choice for band W: CDTW_VARIANT_REGISTER (one thread per window, band
