@@ -514,6 +514,7 @@ def subresults(h, dev, peak=None) -> dict:
         D = torch.empty(n, device=dev)
         gq, gs = torch.empty_like(q), torch.empty_like(s)
         fns = {"fwd": lambda: h.pair_fwd(q, s, W, out=D),
+               "fwd_path_default": lambda: h.pair_fwd(q, s, W, path=path, out=D),
                "fwd_path": lambda: h.pair_fwd(q, s, W, path=path, out=D, mode="store"),
                "fwd_path_recompute": lambda: h.pair_fwd(q, s, W, path=path, out=D,
                                                         mode="recompute"),
@@ -660,8 +661,9 @@ def profile_case(name: str) -> None:
     batch_short = the batched search of 512 queries (M 64-128) on a 2^20 ECG-like
     stream; topk =
     top-1000 of one M=256 template on a 2^22 ECG-like stream; pair = 256 pairs
-    of L=2048, W=409 and 4096 pairs of L=256, W=25 (forward, forward with path,
-    backward); refine = 8 templates x 200 matches, 5 Adam steps; refine_search
+    of L=2048, W=409 and 4096 pairs of L=256, W=25 (forward, forward with path in
+    each mode, backward); ed = the ED profile of 2^21 samples, M=256; ldtw = the
+    LDTW profile of 2^20 samples, M=128, W=12; refine = 8 templates x 200 matches, 5 Adam steps; refine_search
     = the same with random-walk templates and the matches searched at every
     step."""
     import torch
@@ -712,9 +714,19 @@ def profile_case(name: str) -> None:
                                          .astype(np.float32)).to(dev)
                     path = torch.empty(h.pair_path_bytes(n, L), dtype=torch.uint8, device=dev)
                     h.pair_fwd(q, s, W)
+                    h.pair_fwd(q, s, W, path=path)
                     h.pair_fwd(q, s, W, path=path, mode="store")
                     h.pair_fwd(q, s, W, path=path, mode="recompute")
                     h.pair_bwd(q, s, path)
+            elif name == "ed":
+                x = synth.metal_like(1 << 21, seed=1).astype(np.float64)
+                q = x[5000:5256] + 0.1
+                h.ed_all_windows(torch.from_numpy(q).to(dev), torch.from_numpy(x).to(dev))
+            elif name == "ldtw":
+                x = synth.ecg_like(1 << 20, seed=0)
+                q, _ = synth.cut_query(x, 128, seed=5, noise=0.1)
+                h.set_query(q, 12)
+                h.ldtw_ref_all_windows(torch.from_numpy(x).to(dev), 0)
             elif name == "refine":
                 x = synth.ecg_like(1 << 20, seed=0)
                 dx = torch.from_numpy(x).to(dev)
@@ -757,7 +769,7 @@ def main() -> None:
     ap.add_argument("--impl", choices=["ours", "reference"], default="ours")
     ap.add_argument("--profile",
                     choices=["search", "search1024", "topk", "pair", "refine", "refine_search",
-                             "strip", "wide", "wide409", "batch_short"],
+                             "strip", "wide", "wide409", "batch_short", "ed", "ldtw"],
                     help="run one small case of that row twice (for ncu) and exit")
     ap.add_argument("--no-sub", action="store_true",
                     help="skip the pruned / batched search and pair fwd/bwd sub-results")
