@@ -201,7 +201,8 @@ class Handle:
 
     def topk(self, subject, avg, std, k: int, metric=EUCLIDEAN):
         """The k best non-overlapping windows of the query: (locations,
-        distances) best first, distances as the search prints them."""
+        distances) best first, distances as the search prints them; every step
+        on the device."""
         locs = np.empty(k, np.int64)
         dists = np.empty(k, np.float32)
         found = ctypes.c_int()
@@ -211,8 +212,7 @@ class Handle:
         return locs[:found.value], dists[:found.value]
 
     def topk_device(self, subject, avg, std, k: int, metric=EUCLIDEAN):
-        """topk with every step on the device (cdtw_topk_device): the same
-        picks, no host round trip before the end."""
+        """topk by its other name (cdtw_topk_device): the same call."""
         locs = np.empty(k, np.int64)
         dists = np.empty(k, np.float32)
         found = ctypes.c_int()

@@ -43,7 +43,7 @@ __device__ __forceinline__ void copy8(double* dst, const double* src, bool in) {
 // through (tile, query chunk) stages with the next stage's copies in flight
 // under the current one's arithmetic: with a block per tile every wave of
 // blocks loaded together, computed together and divided by sigma together (60
-// us; with the statistics pass 81, now 67).
+// us; with the statistics pass 81, now 57 and 71).
 __global__ void __launch_bounds__(kEdThreads)
 ed_kernel(const double* __restrict__ x, int64_t N, const double* __restrict__ zq, int M,
           int64_t Nw, const double* __restrict__ rs, double* __restrict__ out) {

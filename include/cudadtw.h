@@ -431,7 +431,8 @@ int cdtw_refine_templates_search(cdtw_handle h, const float* d_subject, int64_t 
 
 enum cdtw_variant {
     CDTW_VARIANT_AUTO = 0,      /* built-in rule: register band for W <= 106, lane groups up
-                                   to W = 767, 16-row strips above                      */
+                                   to W = 767, 16-row strips above; at W = 97..106 the
+                                   number of windows decides between the first two      */
     CDTW_VARIANT_REGISTER = 1,  /* one thread per window, the band in registers (W <= 106) */
     CDTW_VARIANT_STRIP16 = 2,   /* strips of 16 rows, boundary ring (W >= 15)            */
     CDTW_VARIANT_STRIP32 = 3,   /* strips of 32 rows, boundary ring (W >= 31)            */
