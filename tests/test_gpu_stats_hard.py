@@ -106,25 +106,34 @@ def test_ed_precision_on_an_ordinary_stream():
     assert np.sqrt(np.square(err).mean()) <= 3.4e-15
 
 
+def _time(h, x, m):
+    d = torch.from_numpy(x).cuda()
+    runs = []
+    for _ in range(8):
+        a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+        a.record()
+        h.avg_std(d, m)
+        b.record()
+        torch.cuda.synchronize()
+        runs.append(a.elapsed_time(b))
+    return min(runs)
+
+
 def test_bad_samples_do_not_serialise_the_pass():
     """A NaN every 3000 samples concerns a thread in 188: at most twice the time
     of a clean stream, with as much again for the clock."""
     from cudadtw_b200 import Handle
-    n, m = 1 << 20, 2000
-    x = synth.ecg_like(n, seed=3)
+    x = synth.ecg_like(1 << 20, seed=3)
     y = x.copy()
     y[::3000] = np.float32(np.nan)
-    took = []
     with Handle(0) as h:
-        for s in (x, y):
-            d = torch.from_numpy(s).cuda()
-            runs = []
-            for _ in range(8):
-                a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
-                a.record()
-                h.avg_std(d, m)
-                b.record()
-                torch.cuda.synchronize()
-                runs.append(a.elapsed_time(b))
-            took.append(min(runs))
-    assert took[1] <= 4.0 * took[0]
+        assert _time(h, y, 2000) <= 4.0 * _time(h, x, 2000)
+
+
+def test_single_samples_take_no_longer_than_short_windows():
+    """Windows of one sample have no variance to lose (each taken again took 2.5
+    times the pass)."""
+    from cudadtw_b200 import Handle
+    x = synth.metal_like(1 << 23, seed=3)
+    with Handle(0) as h:
+        assert _time(h, x, 1) <= 1.3 * _time(h, x, 32)
